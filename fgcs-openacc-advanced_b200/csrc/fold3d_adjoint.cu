@@ -218,17 +218,8 @@ __device__ __forceinline__ bool adj_item(const AdjWaveArgs &b, const EllipParam 
         // in the queue and never publish (nor push)
         if (nu >= 0 && nu < a.ntu && nv >= 0 && nv < a.ntv &&
             b.has[(long long)(tgt + a.sg) * ntiles + nv * a.ntu + nu]) {
-            const unsigned *fl = a.flags + (long long)(p - 1) * ntiles + nv * a.ntu + nu;
-            const unsigned long long t0 = global_ns();
-            unsigned spins = 0;
-            while (ld_acquire(fl) < want) {
-                if (++spins > (1u << 26) || global_ns() - t0 > a.timeout_ns || *(volatile unsigned *)a.status != 0) {
-                    atomicCAS(a.status, 0u, 1u);  // FOLD3D_ERR_TIMEOUT
-                    timed_out = 1;
-                    break;
-                }
-                if (kPollNs) __nanosleep(kPollNs);
-            }
+            timed_out = wait_flag(a.flags + (long long)(p - 1) * ntiles + nv * a.ntu + nu, want, a.status,
+                                  a.timeout_ns) == 0;
         }
     }
     if (__syncthreads_or(timed_out)) return false;
@@ -302,12 +293,8 @@ __global__ void __launch_bounds__(kAdjThreads, 1024 / kAdjThreads) batch_adj_pas
         const int il = (int)(e >> 40), local = (int)(e & ((1ll << 40) - 1));
         __syncthreads();  // every thread has read s_next and s_il
         if (threadIdx.x == 0) {  // claim the next item now; it is processed after this one
-            long long it = -1;
-            if (*(volatile unsigned *)ba.status == 0) {
-                const unsigned w = atomicAdd(ba.work, 1u);
-                if (w < ba.total) it = (long long)ba.items[w];
-            }
-            s_next = it;
+            const unsigned w = atomicAdd(ba.work, 1u);
+            s_next = (w < ba.total) ? (long long)ba.items[w] : -1ll;
         }
         if (il != s_il) {  // consecutive items mostly share their instance
             const unsigned *src = reinterpret_cast<const unsigned *>(ba.inst + il);

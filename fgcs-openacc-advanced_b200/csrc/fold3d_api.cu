@@ -167,6 +167,7 @@ struct fold3d_ctx {
     size_t d_field_cells = 0;
     // WAVEFRONT engine scratch, sized for the grid of key_wg
     fold3d_grid key_wg{};
+    int key_wtv = 0;                         // and tiles of this many rows
     unsigned *w_flags = nullptr;
     unsigned *w_mod[3] = {nullptr, nullptr, nullptr};
     unsigned *w_counters = nullptr;          // [0] work, [1] status
@@ -180,7 +181,8 @@ struct fold3d_ctx {
     std::map<std::vector<long long>, std::pair<int, int>> tuned;  // size mix -> (tile height, CTAs per SM)
     double *tune_T = nullptr;                // autotuner: copies of a few instances' fields
     size_t tune_cells = 0;
-    int wave_bps[2][2][2] = {};              // [ellip][f32][large plane] resident CTAs per SM
+    int wave_bps[2][2] = {};                 // [f32][large plane] resident CTAs per SM, elliptical medium
+    int drift_bps[9] = {};                   // and drift medium, by tile rows
     // batched solves: per-instance scratch and per-direction staging
     std::vector<int> bkey;                   // dims of the instances the scratch is sized for
     unsigned *b_scratch = nullptr;           // flags and change maps of all instances
@@ -379,13 +381,26 @@ static int solve_planes(fold3d_ctx *c, const fold3d_grid &g, const fold3d_medium
     return FOLD3D_OK;
 }
 
-// WAVEFRONT tiles (32 x kWaveTV) per plane of the orientation with normal axis b.
+// WAVEFRONT tiles (32 x tv) per plane of the orientation with normal axis b.
 static void orient_tiles(const fold3d_grid &g, int b, int &ntu, int &ntv, int tv = kWaveTV)
 {
     const int n[3] = {g.nx, g.ny, g.nz};
     const int ub = (b == 0) ? 1 : 0, vb = (b == 2) ? 1 : 2;
     ntu = (n[ub] + 31) / 32;
     ntv = (n[vb] + tv - 1) / tv;
+}
+
+// The change maps of a pass (maps[b]: normal axis b) in the order of WaveArgs.
+static void pass_maps(WaveArgs &a, const fold3d_grid &g, unsigned *const maps[3], int tv)
+{
+    const int axes[3] = {a.nrm, a.ua, a.va};
+    for (int q = 0; q < 3; ++q) {
+        int ntu, ntv;
+        orient_tiles(g, axes[q], ntu, ntv, tv);
+        a.mod[q] = maps[axes[q]];
+        a.mod_ntu[q] = ntu;
+        a.mod_ntiles[q] = ntu * ntv;
+    }
 }
 
 // Pass numbers travel as (pass << 1) | changed in 32-bit flags.  Far before
@@ -409,9 +424,10 @@ static int reserve_passes(fold3d_ctx *c, unsigned passes)
     return FOLD3D_OK;
 }
 
-static int wave_scratch(fold3d_ctx *c, const fold3d_grid &g)
+static int wave_scratch(fold3d_ctx *c, const fold3d_grid &g, int tv)
 {
-    if (c->w_flags && c->key_wg.nx == g.nx && c->key_wg.ny == g.ny && c->key_wg.nz == g.nz) return FOLD3D_OK;
+    if (c->w_flags && c->key_wg.nx == g.nx && c->key_wg.ny == g.ny && c->key_wg.nz == g.nz && c->key_wtv == tv)
+        return FOLD3D_OK;
     if (c->w_flags) cudaFree(c->w_flags);
     for (int b = 0; b < 3; ++b) {
         if (c->w_mod[b]) cudaFree(c->w_mod[b]);
@@ -423,7 +439,7 @@ static int wave_scratch(fold3d_ctx *c, const fold3d_grid &g)
     cudaError_t e;
     for (int b = 0; b < 3; ++b) {
         int ntu, ntv;
-        orient_tiles(g, b, ntu, ntv);
+        orient_tiles(g, b, ntu, ntv, tv);
         flag_words = std::max(flag_words, (size_t)(n[b] - 1) * ntu * ntv);
         const size_t words = (size_t)(n[b] + 2) * ntu * ntv;
         if ((e = cudaMalloc(&c->w_mod[b], words * 4)) != cudaSuccess ||
@@ -443,6 +459,7 @@ static int wave_scratch(fold3d_ctx *c, const fold3d_grid &g)
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, dev);
     }
+    c->key_wtv = tv;
     c->key_wg = g;  // fresh flags and maps are zero, below every pass number to come
     return FOLD3D_OK;
 }
@@ -472,26 +489,34 @@ static EllipParam ellip_param(const fold3d_grid &g, const EllipMedium &m, int di
 }
 
 // T: double, or float when f32 (elliptical medium only).
+// Rows of the drift medium's tiles, from the mean number of 32-point rows in a
+// plane step.  An item's rows run one after another on one warp, so few rows
+// per item keep the plane-to-plane chain short, and many share the cost of a
+// claim, a wait and a publishing fence (about 4000 cycles).  Measured, ms for 3
+// sweeps with 1, 2 and 4 rows: 320^3 (3200 rows a step) 66, 99, 167; 512^3
+// (8192) 126, 166, 279; 640^3 (12800) 281, 270, 415; 896^3 (25088) 819, 617,
+// 705; 1024^3 (32768) 1222, 912, 906; 1280^3 (51200) 2416, 1779, 1549.
+static int drift_tile_rows(const fold3d_grid &g)
+{
+    if (FOLD3D_DRIFT_TV) return FOLD3D_DRIFT_TV;
+    const double rows = 3.0 * g.nx * g.ny * g.nz / 32.0 / ((double)g.nx + g.ny + g.nz);
+    return rows < 12000.0 ? 1 : rows < 32000.0 ? 2 : 4;
+}
+
 static int solve_wavefront(fold3d_ctx *c, const fold3d_grid &g, const fold3d_medium *fm, const EllipMedium *em,
                            void *T, bool f32, const fold3d_opts &o, cudaStream_t s, fold3d_report *rep,
                            unsigned char *winners = nullptr)
 {
     int rc = reserve_passes(c, 6u * (unsigned)std::min(o.max_sweeps, 1 << 20) + 12u);
     if (rc) return rc;
-    if ((rc = wave_scratch(c, g))) return rc;
+    const int tv = em ? kWaveTV : drift_tile_rows(g);
+    if ((rc = wave_scratch(c, g, tv))) return rc;
     cudaError_t e;
     if ((e = cudaMemsetAsync(c->w_counters, 0, 2 * sizeof(unsigned), s)) != cudaSuccess ||
         (e = cudaMemsetAsync(c->w_evaluated, 0, sizeof(unsigned long long), s)) != cudaSuccess)
         return cuda_error(e, "cudaMemsetAsync");
     WaveArgs a;
     memset(&a, 0, sizeof a);
-    for (int b = 0; b < 3; ++b) {
-        int ntu, ntv;
-        orient_tiles(g, b, ntu, ntv);
-        a.mod[b] = c->w_mod[b];
-        a.mod_ntu[b] = ntu;
-        a.mod_ntiles[b] = ntu * ntv;
-    }
     a.flags = c->w_flags;
     a.work = c->w_counters;
     a.status = c->w_counters + 1;
@@ -515,7 +540,8 @@ static int solve_wavefront(fold3d_ctx *c, const fold3d_grid &g, const fold3d_med
             a.ua = (d.nrm == 0) ? 1 : 0;
             a.va = (d.nrm == 2) ? 1 : 2;
             a.sg = d.sg;
-            orient_tiles(g, d.nrm, a.ntu, a.ntv);
+            orient_tiles(g, d.nrm, a.ntu, a.ntv, tv);
+            pass_maps(a, g, c->w_mod, tv);
             a.steps = pass_count(a.pg);
             a.first_src = pass_first(a.pg, dir);
             a.epoch = ++c->epoch;
@@ -523,16 +549,19 @@ static int solve_wavefront(fold3d_ctx *c, const fold3d_grid &g, const fold3d_med
             a.winners = winners;
             const long long items = (long long)a.steps * a.ntu * a.ntv;
             const bool large = (long long)a.ntu * a.ntv >= kLargePlaneTiles;
-            int &bps = c->wave_bps[em ? 1 : 0][f32 ? 1 : 0][large ? 1 : 0];
-            if (!bps) bps = wave_blocks_per_sm(em ? kMediumEllip : kMediumDrift, f32, large);
-            const int grid = (int)std::min<long long>(items, (long long)c->sms * bps);
+            int &bps = em ? c->wave_bps[f32 ? 1 : 0][large ? 1 : 0] : c->drift_bps[tv];
+            if (!bps) bps = em ? wave_blocks_per_sm(f32, large) : drift_blocks_per_sm(tv);
+            const long long ctas = em ? items : (items + 3) / 4;  // the drift medium's warps take items of their own
+            const int grid = (int)std::min<long long>(ctas,
+                                                      (long long)c->sms * bps);
             if ((e = cudaMemsetAsync(a.work, 0, sizeof(unsigned), s)) != cudaSuccess)
                 return cuda_error(e, "cudaMemsetAsync");
             if (em) {
                 e = launch_wave_pass_ellip(T, f32, a, ellip_param(g, *em, dir), grid, s, large);
             } else {
                 build_dir_table(make_frame(g, *fm, dir), tab);
-                e = launch_wave_pass(static_cast<double *>(T), a, tab, grid, s, large);
+                orient_table(tab, d.xa == a.ua, d.xs, d.ys);
+                e = launch_wave_pass(static_cast<double *>(T), a, tab, tv, grid, s);
             }
             if (e != cudaSuccess) return cuda_error(e, "wavefront pass");
         }
@@ -785,13 +814,9 @@ static int solve_batch_cfg(fold3d_ctx *c, int n, const SolveInst *in, bool f32, 
             a.first_src = pass_first(a.pg, dir);
             a.timeout_ns = 4000000000ull;
             a.flags = c->b_scratch + c->b_flag_off[i];
-            for (int b = 0; b < 3; ++b) {
-                int ntu, ntv;
-                orient_tiles(g, b, ntu, ntv, tv);
-                a.mod[b] = c->b_scratch + c->b_mod_off[b][i];
-                a.mod_ntu[b] = ntu;
-                a.mod_ntiles[b] = ntu * ntv;
-            }
+            unsigned *const maps[3] = {c->b_scratch + c->b_mod_off[0][i], c->b_scratch + c->b_mod_off[1][i],
+                                       c->b_scratch + c->b_mod_off[2][i]};
+            pass_maps(a, g, maps, tv);
             a.work = c->b_counters;
             a.status = c->b_counters + 1;
             a.maxd = c->b_slots + i;
@@ -1557,7 +1582,8 @@ int fold3d_selftest_wait_timeout(fold3d_ctx *c, double timeout_ms)
     DeviceGuard dg(c->device);
     const fold3d_grid g = {16, 16, 16, 1.0, 1.0, 1.0};
     const fold3d_medium m = {1.1, -0.35, 0.4, 0.7};
-    int rc = wave_scratch(c, g);
+    const int tv = drift_tile_rows(g);
+    int rc = wave_scratch(c, g, tv);
     if (rc) return rc;
     cudaError_t e;
     const size_t cells = field_cells(g);
@@ -1573,13 +1599,6 @@ int fold3d_selftest_wait_timeout(fold3d_ctx *c, double timeout_ms)
     cudaStream_t s = c->stream;
     WaveArgs a;
     memset(&a, 0, sizeof a);
-    for (int b = 0; b < 3; ++b) {
-        int ntu, ntv;
-        orient_tiles(g, b, ntu, ntv);
-        a.mod[b] = c->w_mod[b];
-        a.mod_ntu[b] = ntu;
-        a.mod_ntiles[b] = ntu * ntv;
-    }
     a.flags = c->w_flags;
     a.work = c->w_counters;
     a.status = c->w_counters + 1;
@@ -1592,17 +1611,19 @@ int fold3d_selftest_wait_timeout(fold3d_ctx *c, double timeout_ms)
     a.ua = 0;
     a.va = 1;
     a.sg = 1;
-    orient_tiles(g, 2, a.ntu, a.ntv);
+    orient_tiles(g, 2, a.ntu, a.ntv, tv);
+    pass_maps(a, g, c->w_mod, tv);
     a.steps = pass_count(a.pg);
     a.first_src = 1;
     a.epoch = ++c->epoch;
     DirTable tab;
     build_dir_table(make_frame(g, m, FOLD3D_K_UP), tab);
+    orient_table(tab, kDirs[FOLD3D_K_UP].xa == a.ua, kDirs[FOLD3D_K_UP].xs, kDirs[FOLD3D_K_UP].ys);
     // start the item counter after step 0: step 1 then waits for flags nothing sets
     const unsigned start[2] = {(unsigned)(a.ntu * a.ntv), 0u};
     unsigned hstat[2] = {0, 0};
     if ((e = cudaMemcpyAsync(c->w_counters, start, sizeof start, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-        (e = launch_wave_pass(c->d_field, a, tab, 4, s)) != cudaSuccess ||
+        (e = launch_wave_pass(c->d_field, a, tab, tv, 4, s)) != cudaSuccess ||
         (e = cudaMemcpyAsync(hstat, c->w_counters, sizeof hstat, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
         (e = cudaStreamSynchronize(s)) != cudaSuccess)
         return cuda_error(e, "selftest");

@@ -27,12 +27,15 @@
 //    spacings and bounded slowness terms).
 //
 // Data-dependent square roots and the two divisions by data-dependent
-// values keep CUDA's IEEE operations.  The candidate bodies run as loops over
-// table slots instead of 24 inlined copies, which keeps the kernel small.
-// Because each solver call only accepts candidates strictly below the
-// current time, and every gate that depends on the current time only skips
-// calls that could not lower it, the update is min(T_old, candidates), so the
-// slot loop may visit the calls in any order; it keeps the reference's order.
+// values keep CUDA's IEEE operations.  Each solver call only accepts
+// candidates strictly below the current time, and the calls' own gates on the
+// current time only skip calls that could not lower it, so the calls may be
+// visited in any order.  One gate of the reference is different: its early
+// exit (:231) leaves all sixteen calls out when the time after the 1-D
+// candidate is below seven of the nine sources, xnt and ynt not among them.
+// It is kept as it is.  (Evaluating a point again with the same sources still
+// changes nothing: its time has only fallen, so the exit is taken again
+// wherever it was, and elsewhere the same candidates are not below it.)
 //
 // 3. One more such gate skips a FoldSurf3Points body (its nested edge still
 //    runs) when the current time is at most min(s0, s1, s2) + B.  The body
@@ -68,6 +71,41 @@
 //    the body's single gradient d (fold3d_tables.cpp), less the same
 //    relative 1e-3 margin.  The fall-back candidate from s1 alone is not
 //    gated.
+//
+// 5. Gates and bodies in float first.  A body that passes its gate costs 100
+//    to 150 FP64 instructions of which most depend on one another, and in a
+//    settled field it nearly always ends in a rejection: over 192^3 sweeps of
+//    the reference's workload a warp row enters 4.5 bodies and 0.17 of its
+//    points improve; with the filter it enters 0.4.  So every gate and every body is first judged in float,
+//    from differences rounded once: c_r = float(st - s_r), E = float(tn - st).
+//
+//    Gates.  tn - min(sources) = E + max(c), so a call can only matter when
+//    E + max(c) > B (its skip bound; an edge's fall-back when E + c > K,
+//    covered by taking min(B, K)).  E is raised by 4e-7 |E|, more than the
+//    roundings of E, c and the sum where the two are about equal, and the
+//    thresholds are rounded down, so no call that could matter is dropped.
+//    The calls' fixed early returns (:71, :132, :170) are signs of c and of
+//    c_r - c_s, which rounding never turns into a false return.
+//
+//    Bodies.  Scaled by F (u = F dx, v = F dy, a/F) the triangle's body is
+//    al = 1 - a.(u,v), q = al^2 - g(u^2 + v^2), S = sqrt q,
+//    z = (S - az al)/g, w = al - az z (= F|p| while F > |a|), and the ray is
+//    (u + ax w, v + ay w, S): its time and its four footpoint tests need one
+//    square root and no division.  An edge is the same in two dimensions, with
+//    the reference's own footpoint direction (4. above).  A rejection counts
+//    only if it is clear by m = eps (1 + u^2 + v^2 + al^2)/S, eps = 1e-3.
+//    Bound on the errors, M^2 = 1 + u^2 + v^2 + al^2 and spacings within a
+//    factor of 8 of each other: u and v are off by 2e-6 M (their c by 2^-24
+//    relative, |c| F/h <= 20 M; for a nested edge M^2 also holds
+//    (c F/(4h))^2), al by 8e-6 M, q by 4e-5 M^2, so S by 2e-5 M^2/S; with
+//    F^2 >= 1.1 |a|^2 (az^2/g <= 10) z, w and the ray are then off by at most
+//    3.2e-4 M^2/S, a third of m.  Other media and spacings set eps = +inf,
+//    which rejects nothing, and a non-finite value makes m infinite or NaN,
+//    which rejects nothing either.  What is left goes through the FP64 bodies
+//    with all their gates, so the result is the same bits; a footpoint that
+//    the filter finds inside by m on all sides is not tested again, and a
+//    certain acceptance (its time above all sources' by m too) lowers the
+//    bound that later bodies are judged against.
 #pragma once
 #include <cstdint>
 #include <cstring>
@@ -99,8 +137,58 @@ struct SurfK {
     EdgeK nest;         // the nested FoldEdge2Points call (:172-173)
 };
 
+// Float constants of the filter (5. above) of one FoldSurf3Points body and of
+// one FoldEdge2Points call, in the order the kernels read them (16-byte
+// loads).  Drifts are divided by the body's speed (F, or F' = sqrt(F^2 -
+// ay^2) for an edge), slownesses multiplied by it.
+struct alignas(16) TriF {
+    float kx, ky;      // F/dxx, F/dyy
+    float ax, ay;      // drift / F
+    float r1, r2;      // dyy/(dxx+dyy), dxx/(dxx+dyy)
+    float s1, s2;      // dzz/(dxx+dzz), dxx/(dxx+dzz)
+};
+struct alignas(16) EdgeF {
+    float k, kz;       // F'/dxx, F'/dzz
+    float ax, az;      // drift / F'
+    float ga, iga;     // 1 - az^2, 1/(1 - az^2)
+    float fx, fz;      // F ax, F az: the drift in the footpoint's direction (4. above)
+    float s1, s2;      // dzz/(dxx+dzz), dxx/(dxx+dzz)
+    float ka;          // 1 + |fx| + |fz|
+    float K;           // fall-back increment, rounded down; +inf where it is undefined
+};
+
+// Sources of a target point: the rim of the fan in order xt, txy, yt, tym,
+// xnt, txnyn, ynt, txm (0..7) and st (8).  The sources of call k of the
+// eight FoldSurf3Points (:233-240), four bits each, k = 0 lowest.
+constexpr unsigned kTriS1 = 0x22664400u;  // xt xt xnt xnt ynt ynt yt yt
+constexpr unsigned kTriS2 = 0x31753571u;  // txy txm txnyn tym txnyn txm txy tym
+
+// The filter's constants of one side (5. above).  Call k of the bit masks and
+// thresholds is triangle k, nested edge 8 + k, outer edge 16 + k.  Built in
+// the direction's local frame; orient_table() turns it into the frame of the
+// plane's two axes for the kernels that walk a plane's rows.
+struct alignas(16) SideFilter {
+    float gB[24];             // thresholds of the gates, rounded down
+    float outer;              // the smallest of gB
+    float eps;                // margin, +inf where the bodies are not filtered
+    float faz, fg, fig, fkz;  // az/F, 1 - faz^2, 1/fg, F/dzz
+    float fhz;                // dzz/F, rounded up
+    unsigned every;           // calls that are never gated (all of them, or none)
+    // the calls' fixed early returns as bit masks, bit k for call k
+    unsigned m_e1, m_e2;      // surf[k].e1, .e2
+    unsigned m_nest_early;    // surf[k].nest.early
+    unsigned m_edge_early;    // edge[k].early
+    int d1_ok;                // 1-D candidate
+    int named[2];             // rim points that the early exit (:231) names: 0 or 4, and 2 or 6
+    double K1;
+    // the FP64 constants' entries of triangle k and outer edge k (orient_table)
+    unsigned char surf_at[8], edge_at[8];
+    TriF tri[8];
+    EdgeF ef[16];             // nested edges, then outer edges
+};
+
 // All constants of one direction on one side of the source surface.
-struct SideTable {
+struct alignas(16) SideTable {
     double F, az, hz;
     double g, rg;       // F*F - az*az, RN(1/g)          (:147)
     double K1;          // 1-D candidate increment dzz*dzz/q (:225)
@@ -111,11 +199,17 @@ struct SideTable {
     unsigned m_edge_early;          // edge[k].early
     SurfK surf[8];      // the eight FoldSurf3Points calls (:233-240), in order
     EdgeK edge[8];      // the eight FoldEdge2Points calls (:242-253), in order
+    SideFilter flt;     // the float filter (5. above)
 };
 
 struct DirTable {
     SideTable side[2];  // [0]: target >= 0 (or 0), [1]: target < 0 (drift negated)
 };
+
+// The filter's parts of a table turned from the local frame into the frame of
+// the plane's axes u and v (rim point 0 at u + 1, 2 at v + 1): x_is_u, the
+// local x axis is u; xs, ys, the signs of the local axes.
+void orient_table(DirTable &tab, bool x_is_u, int xs, int ys);
 
 // Safe operand range of div_by_const: |x| and |c| in [2^-400, 2^401), which
 // keeps the quotient, the products and the remainders normal.  The host
@@ -154,83 +248,342 @@ __host__ __device__ __forceinline__ double div_by_const(double x, double c, doub
 
 __host__ __device__ __forceinline__ double kmin(double a, double b) { return (a < b) ? a : b; }
 
-__host__ __device__ __forceinline__ void edge_k(double &tn, double s0, double s1, const EdgeK &k, double F)
+// Fixed early returns: of a FoldSurf3Points call (:132), of its nested
+// FoldEdge2Points call (:170, :71, behind the former), of an outer one (:71).
+__host__ __device__ __forceinline__ bool surf_closed(double s0, double s1, double s2, const SurfK &k)
+{
+    return ((k.e1 != 0) & (s1 > s0)) | ((k.e2 != 0) & (s2 > s1));
+}
+__host__ __device__ __forceinline__ bool nest_closed(double s0, double s1, double s2, const SurfK &k)
+{
+    return surf_closed(s0, s1, s2, k) | ((k.nblock != 0) & (s1 > s2)) | ((k.nest.early != 0) & (s2 > s1));
+}
+
+// FoldEdge2Points' own body (:75-97).  inside: the footpoint is known to lie
+// on the edge (5. below), so its test is left out.
+__host__ __device__ __forceinline__ void edge_body(double &tn, double s0, double s1, const EdgeK &k, double F,
+                                                   bool inside)
 {
     const double mn = kmin(s1, s0);
-    if (tn < mn || (k.early && s1 > s0)) return;
-    if (!(tn <= mn + k.B)) {  // 4. above
-        const double d = div_by_const(s1 - s0, k.hx, k.rhx);
-        double c = (1.0 - d * k.ax);
-        double q = k.g * (c * c - d * d * k.ga);
-        if (0.0 < q) {
-            c = div_by_const(-k.az * c + sqrt(q), k.ga, k.rga);
-            q = s0 + k.hz * c;
-            if (q < tn && q > mn) {
-                const double g = sqrt(div_by_const((d * d + c * c) * F * F, k.g, k.rg));
-                const double xe = -k.hz * (d + k.ax * g) / (c + k.az * g);
-                if (0.0 < xe && xe < k.hx) tn = q;
-            }
-        }
+    if (tn <= mn + k.B) return;  // 4. above
+    const double d = div_by_const(s1 - s0, k.hx, k.rhx);
+    double c = (1.0 - d * k.ax);
+    double q = k.g * (c * c - d * d * k.ga);
+    if (!(0.0 < q)) return;
+    c = div_by_const(-k.az * c + sqrt(q), k.ga, k.rga);
+    q = s0 + k.hz * c;
+    if (!(q < tn && q > mn)) return;
+    if (!inside) {
+        const double g = sqrt(div_by_const((d * d + c * c) * F * F, k.g, k.rg));
+        const double xe = -k.hz * (d + k.ax * g) / (c + k.az * g);
+        if (!(0.0 < xe && xe < k.hx)) return;
     }
-    if (tn > s1 && k.fb_ok) tn = kmin(tn, s1 + k.K);
+    tn = q;
 }
 
-__host__ __device__ __forceinline__ void surf_k(double &tn, double s0, double s1, double s2, const SurfK &k,
-                                                const SideTable &t)
+// FoldSurf3Points' own body (:131-165); inside as above.
+__host__ __device__ __forceinline__ void surf_body(double &tn, double s0, double s1, double s2, const SurfK &k,
+                                                   const SideTable &t, bool inside)
 {
     const double mn = kmin(s0, kmin(s1, s2));
-    if (tn < mn || (k.e1 && s1 > s0) || (k.e2 && s2 > s1)) return;
-    if (!(tn <= mn + k.B)) {  // 3. above
-        const double dx = div_by_const(s1 - s0, k.hx, k.rhx);
-        const double dy = div_by_const(s2 - s1, k.hy, k.rhy);
-        double dd = dx * dx + dy * dy;
-        double al = 1.0 - k.ax * dx - k.ay * dy;
-        double q = al * al - dd * t.g;
-        if (q > 0.0) {
-            al = div_by_const(-t.az * al + t.F * sqrt(q), t.g, t.rg);
-            const double g = s0 + t.hz * al;
-            if (g < tn && g > mn) {
-                q = sqrt(dd + al * al);
-                dd = -t.hz / (t.F * al + t.az * q);
-                const double xe = dd * (t.F * dx + k.ax * q);
-                const double ye = dd * (t.F * dy + k.ay * q);
-                if (0.0 <= kmin(xe, ye) && ye * k.hx <= xe * k.hy && xe <= k.hx) tn = g;
-            }
-        }
+    if (tn <= mn + k.B) return;  // 3. above
+    const double dx = div_by_const(s1 - s0, k.hx, k.rhx);
+    const double dy = div_by_const(s2 - s1, k.hy, k.rhy);
+    double dd = dx * dx + dy * dy;
+    double al = 1.0 - k.ax * dx - k.ay * dy;
+    double q = al * al - dd * t.g;
+    if (!(q > 0.0)) return;
+    al = div_by_const(-t.az * al + t.F * sqrt(q), t.g, t.rg);
+    const double g = s0 + t.hz * al;
+    if (!(g < tn && g > mn)) return;
+    if (!inside) {
+        q = sqrt(dd + al * al);
+        dd = -t.hz / (t.F * al + t.az * q);
+        const double xe = dd * (t.F * dx + k.ax * q);
+        const double ye = dd * (t.F * dy + k.ay * q);
+        if (!(0.0 <= kmin(xe, ye) && ye * k.hx <= xe * k.hy && xe <= k.hx)) return;
     }
-    if (tn > kmin(s1, s2) && !(k.nblock && s1 > s2)) edge_k(tn, s1, s2, k.nest, t.F);
+    tn = g;
 }
 
-// New signed value of a target whose stored value is `told`, from the nine
-// previous-plane magnitudes (named as in the reference, :195-204).
-__host__ __device__ __forceinline__ double point_update_fast(double told, double st, double xt, double yt,
-                                                             double xnt, double ynt, double txy, double txm,
-                                                             double tym, double txnyn, const DirTable *tab)
+// ---------------------------------------------------------------------------
+// The float filter (5. above) and the point update built on it.  On the
+// device a warp's lanes hold 32 points and the calls are visited for all of
+// them together: the warp walks the union of its lanes' calls, so call
+// numbers and table addresses are uniform, and an FP64 body runs only when
+// some lane needs it.  On the host a "warp" is one point.
+// ---------------------------------------------------------------------------
+__host__ __device__ __forceinline__ bool lanes_any(bool p)
 {
+#ifdef __CUDA_ARCH__
+    return __any_sync(0xffffffffu, p);
+#else
+    return p;
+#endif
+}
+
+__host__ __device__ __forceinline__ unsigned lanes_or(unsigned m)
+{
+#ifdef __CUDA_ARCH__
+    return __reduce_or_sync(0xffffffffu, m);
+#else
+    return m;
+#endif
+}
+
+// 1/sqrt(x) to a few ulp, x normal and > 0.
+__host__ __device__ __forceinline__ float filter_rsqrt(float x)
+{
+#ifdef __CUDA_ARCH__
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+#else
+    return 1.0f / sqrtf(x);
+#endif
+}
+
+// m with the sign bit of x appended.
+__host__ __device__ __forceinline__ unsigned push_sign(unsigned m, float x)
+{
+#ifdef __CUDA_ARCH__
+    return __funnelshift_l(__float_as_uint(x), m, 1);
+#else
+    uint32_t b;
+    std::memcpy(&b, &x, sizeof b);
+    return (m << 1) | (b >> 31);
+#endif
+}
+
+// 16-byte loads of a call's constants.
+template <class K> __host__ __device__ __forceinline__ K load_consts(const K &k)
+{
+    static_assert(sizeof(K) % 16 == 0, "whole 16-byte words");
+    K r;
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(K) / 16); ++i) reinterpret_cast<float4 *>(&r)[i] = reinterpret_cast<const float4 *>(&k)[i];
+    return r;
+}
+
+// What the filter says of a body: it certainly cannot lower the time, its
+// footpoint is certainly inside, or neither.
+enum Verdict { kNever = 0, kPerhaps = 1, kInside = 3 };
+
+// A triangle's body.  E: a bound of the new time above st; lowered when the
+// body is certain to accept a smaller one.
+__host__ __device__ __forceinline__ unsigned tri_may(float &E, float c1, float c2, const TriF &k, const SideFilter &t)
+{
+    const float u = -c1 * k.kx, v = (c1 - c2) * k.ky;
+    const float al = fmaf(-k.ay, v, fmaf(-k.ax, u, 1.0f));
+    const float dd = fmaf(u, u, v * v);
+    const float sc = t.eps * fmaf(al, al, dd + 1.0f);
+    const float q = fmaf(al, al, -(t.fg * dd));
+    const float qp = fmaxf(q, 1e-20f);
+    const float rs = filter_rsqrt(qp), S = qp * rs;
+    const float z = fmaf(-t.faz, al, S) * t.fig;
+    const float w = fmaf(-t.faz, z, al);
+    const float nx = fmaf(k.ax, w, u), ny = fmaf(k.ay, w, v);
+    const float late = fmaf(-E, t.fkz, z);                                      // later than the time
+    const float diag = fmaf(nx, k.r1, -(ny * k.r2)), far = -fmaf(nx, k.s1, S * k.s2);  // beyond the far sides
+    const float out = fmaxf(fmaxf(nx, ny), fmaxf(diag, far)), m = sc * rs;
+    const bool never = fmaxf(out, late) > m || q < -0.04f * sc;
+    const bool inside = out < -m && q > 0.04f * sc && z > m && v != 0.0f;  // v = 0: :132 is undecided
+    if (inside) E = fminf(E, (z + m) * t.fhz);
+    return never ? kNever : inside ? kInside : kPerhaps;
+}
+
+// An edge's body; ca, cb: c of its two sources.
+__host__ __device__ __forceinline__ unsigned edge_may(float &E, float ca, float cb, const EdgeF &k, const SideFilter &t)
+{
+    const float u = (ca - cb) * k.k, b = 0.25f * ca * k.k;
+    const float c0 = fmaf(-k.ax, u, 1.0f);
+    const float uu = u * u;
+    const float sc = t.eps * fmaf(b, b, fmaf(c0, c0, uu + 1.0f));
+    const float q = fmaf(c0, c0, -(k.ga * uu));
+    const float qp = fmaxf(q, 1e-20f);
+    const float rs = filter_rsqrt(qp), S = qp * rs;
+    const float z = fmaf(-k.az, c0, S) * k.iga;
+    const float m = sc * rs, mk = m * k.ka;
+    const float late = fmaf(-(E + ca), k.kz, z);
+    const float w = fmaf(-k.az, z, c0);
+    const float nx = fmaf(k.fx, w, u), nz = fmaf(k.fz, w, z);
+    const float far = fmaf(fabsf(nx), k.s1, -(fabsf(nz) * k.s2));     // |xe| > dxx
+    const float same = fmaxf(fminf(nx, nz), -fmaxf(nx, nz));          // > 0: one sign, xe < 0
+    const float out = fmaxf(far, same);
+    const bool never = late > m || out > mk || q < -0.04f * sc;
+    const bool inside = out < -mk && q > 0.04f * sc && z > m;
+    return never ? kNever : inside ? kInside : kPerhaps;
+}
+
+// The calls that could lower a point's time after its 1-D candidate, as a bit
+// mask; c: float(st - s_r) of the rim, E: float(tn - st).
+__host__ __device__ __forceinline__ unsigned gate_mask(const float c[8], float E, const SideFilter &t)
+{
+    float gB[24];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        const float4 b = reinterpret_cast<const float4 *>(t.gB)[i];
+        gB[4 * i] = b.x;
+        gB[4 * i + 1] = b.y;
+        gB[4 * i + 2] = b.z;
+        gB[4 * i + 3] = b.w;
+    }
+    const float Eu = fmaf(fabsf(E), 4e-7f, E);
+    const float m01 = fmaxf(c[0], c[1]), m12 = fmaxf(c[1], c[2]), m23 = fmaxf(c[2], c[3]), m34 = fmaxf(c[3], c[4]),
+                m45 = fmaxf(c[4], c[5]), m56 = fmaxf(c[5], c[6]), m67 = fmaxf(c[6], c[7]), m70 = fmaxf(c[7], c[0]);
+    const float X[8] = {m01, m70, m45, m34, m56, m67, m12, m23};  // per triangle, the larger of its rim points
+    // the sign bits of threshold - (time - smallest source); four independent
+    // chains of shifts
+    unsigned spokes = 0, nests = 0, tris = 0, up2 = 0, spoke = 0;
+    constexpr int S1[8] = {0, 0, 4, 4, 6, 6, 2, 2}, S2[8] = {1, 7, 5, 3, 5, 7, 1, 3};
+#pragma unroll
+    for (int k = 7; k >= 0; --k) {
+        tris = push_sign(tris, gB[k] - (Eu + fmaxf(X[k], 0.0f)));
+        nests = push_sign(nests, gB[8 + k] - (Eu + X[k]));
+        spokes = push_sign(spokes, gB[16 + k] - (Eu + fmaxf(c[k], 0.0f)));
+        // fixed early returns: bit k of up2: s2 > s1 (per triangle), of spoke: s_r > st
+        spoke = push_sign(spoke, c[k]);
+        up2 = push_sign(up2, c[S2[k]] - c[S1[k]]);
+    }
+    // bit k of up1: s1 > st
+    const unsigned up1 = (spoke & 1u) * 0x03u | ((spoke >> 4) & 1u) * 0x0cu | ((spoke >> 6) & 1u) * 0x30u |
+                         ((spoke >> 2) & 1u) * 0xc0u;
+    const unsigned gone = (t.m_e1 & up1) | (t.m_e2 & up2);
+    return (tris & ~gone) | ((nests & ~(gone | (t.m_nest_early & up2))) << 8) | ((spokes & ~(t.m_edge_early & spoke)) << 16);
+}
+
+__host__ __device__ __forceinline__ int low_bit(unsigned m)
+{
+#ifdef __CUDA_ARCH__
+    return __ffs((int)m) - 1;
+#else
+    return __builtin_ctz(m);
+#endif
+}
+
+// New signed value of a target whose stored value is `told` from the nine
+// previous-plane magnitudes `s` (rim order, st last).  Every lane of the warp
+// calls it; a lane that is not `active` changes nothing.  sh, ch: scratch of
+// nine doubles and nine floats of this point, `stride` elements apart (shared
+// memory on the device: the walks index the sources by call); tab in shared
+// memory too, since lanes read different calls' constants.
+//
+// The warp walks the union of its lanes' gated calls with the float filter,
+// and each lane notes the bodies that it needs; then every lane runs its own
+// list, so a warp runs as many FP64 bodies as its longest lane's list, not as
+// the lanes' union.
+__host__ __device__ __forceinline__ double point_update_fan(bool active, double told, const double (&s)[9],
+                                                            const DirTable &tab, double *sh, float *ch, int stride)
+{
+    const double st = s[8];
     double tn = fabs(told);
-    const SideTable &t = tab->side[told < 0 ? 1 : 0];
-    if (st < tn && t.d1_ok) tn = kmin(tn, st + t.K1);
-    if (!(tn < st && tn < kmin(xt, yt) && tn < kmin(txy, txm) && tn < kmin(txnyn, tym))) {
-#pragma unroll 1
-        for (int k = 0; k < 8; ++k) {
-            // (xt,txy) (xt,txm) (xnt,txnyn) (xnt,tym) (ynt,txnyn) (ynt,txm) (yt,txy) (yt,tym)
-            const double s1 = (k < 2) ? xt : (k < 4) ? xnt : (k < 6) ? ynt : yt;
-            const int m = k & 3;
-            const double s2 = (m == 0) ? ((k < 4) ? txy : txnyn)
-                            : (m == 1) ? txm
-                            : (m == 2) ? ((k < 4) ? txnyn : txy)
-                                       : tym;
-            surf_k(tn, st, s1, s2, t.surf[k], t);
+    const SideTable &t = tab.side[told < 0 ? 1 : 0];
+    const SideFilter &f = t.flt;
+    float c[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        c[r] = (float)(st - s[r]);
+        sh[r * stride] = s[r];
+        ch[r * stride] = c[r];
+    }
+    sh[8 * stride] = st;
+    ch[8 * stride] = 0.0f;
+    if (st < tn && f.d1_ok) tn = kmin(tn, st + f.K1);
+    float E = (float)(tn - st);
+    const bool odd = !(E > -3e38f) || f.every;  // st infinite or beyond float, or a NaN: gate nothing
+    const float mx = fmaxf(fmaxf(fmaxf(fmaxf(c[0], c[1]), fmaxf(c[2], c[3])), fmaxf(fmaxf(c[4], c[5]), fmaxf(c[6], c[7]))),
+                           0.0f);
+    if (lanes_any(active && (odd || fmaf(fabsf(E), 4e-7f, E) + mx > f.outer))) {
+        unsigned mask = gate_mask(c, E, f);
+        if (odd) mask = 0xffffffu;
+        // the reference's early exit (:231), on the sources it names (not xnt
+        // and ynt): a gate of its own, so judged in FP64 where float is unsure
+        const float lead = E + fmaxf(fmaxf(fmaxf(f.named[0] ? c[4] : c[0], f.named[1] == 2 ? c[2] : c[6]), fmaxf(c[1], c[7])),
+                                     fmaxf(c[5], c[3]));
+        const float unsure = 4e-7f * fabsf(E);
+        if (tn < st && mask && !(lead > unsure)) {
+            if (lead < -unsure || (tn < kmin(sh[f.named[0] * stride], sh[f.named[1] * stride]) &&
+                                   tn < kmin(sh[1 * stride], sh[7 * stride]) &&
+                                   tn < kmin(sh[5 * stride], sh[3 * stride])))
+                mask = 0;
         }
-#pragma unroll 1
-        for (int k = 0; k < 8; ++k) {
-            // xt, txy, yt, tym, xnt, txnyn, ynt, txm
-            const double s1 = (k == 0) ? xt : (k == 1) ? txy : (k == 2) ? yt : (k == 3) ? tym
-                            : (k == 4) ? xnt : (k == 5) ? txnyn : (k == 6) ? ynt : txm;
-            edge_k(tn, st, s1, t.edge[k], t.F);
+        if (!active) mask = 0;
+        // The filter, a triangle and an edge at a time (two chains to overlap).
+        unsigned need = 0, in = 0;  // bodies to run, and those with their footpoint known inside
+        float Eb = odd ? E : fmaf(fabsf(E), 1e-6f, E);  // bound of the new time above st
+        const unsigned all = lanes_or(mask);
+        for (unsigned wt = all & 0xffu, we = all >> 8; wt | we; wt &= wt - 1, we &= we - 1) {
+            const int k = wt ? low_bit(wt) : 0, j = we ? low_bit(we) : 0;
+            const int i1 = (kTriS1 >> (4 * k)) & 15, i2 = (kTriS2 >> (4 * k)) & 15;
+            const int ia = (j < 8) ? (int)((kTriS1 >> (4 * j)) & 15) : 8;
+            const int ib = (j < 8) ? (int)((kTriS2 >> (4 * j)) & 15) : j - 8;
+            const float ca = ch[ia * stride], cb = ch[ib * stride];
+            const EdgeF ef = load_consts(f.ef[j]);
+            const TriF tf = load_consts(f.tri[k]);
+            const bool fall = ((mask >> (8 + j)) & 1u) && (odd || fmaf(fabsf(Eb), 4e-7f, Eb) + cb > ef.K);
+            float Ee = Eb, Et = ((mask >> k) & 1u) ? Eb : -HUGE_VALF;
+            const unsigned ve = edge_may(Ee, ca, cb, ef, f);
+            const unsigned vt = tri_may(Et, ch[i1 * stride], ch[i2 * stride], tf, f);
+            need |= ((vt & 1u) << k) | ((ve & 1u) << (8 + j));
+            in |= ((vt >> 1) << k) | ((ve >> 1) << (8 + j));
+            if ((mask >> k) & 1u) Eb = fminf(Eb, Et);
+            if (fall) {  // the edge's fall-back, :99-113
+                const SurfK &sk = t.surf[f.surf_at[j & 7]];
+                const EdgeK &e = (j < 8) ? sk.nest : t.edge[f.edge_at[j & 7]];
+                const double sa = sh[ia * stride], sb = sh[ib * stride], v = sb + e.K;
+                const bool closed = (j < 8) ? nest_closed(st, sa, sb, sk) : ((e.early != 0) & (sb > st));
+                if ((e.fb_ok != 0) & !closed & (tn > sb) & (v < tn)) {
+                    tn = v;
+                    const float En = (float)(tn - st);
+                    Eb = fminf(Eb, fmaf(fabsf(En), 1e-6f, En));
+                }
+            }
+        }
+        if (odd) need = mask;
+        need &= mask;
+        while (lanes_any((need & 0xffu) != 0)) {
+            if (need & 0xffu) {
+                const int k = low_bit(need);
+                need &= need - 1;
+                const double s1 = sh[((kTriS1 >> (4 * k)) & 15) * stride], s2 = sh[((kTriS2 >> (4 * k)) & 15) * stride];
+                const SurfK &sk = t.surf[f.surf_at[k]];
+                if (!surf_closed(st, s1, s2, sk)) surf_body(tn, st, s1, s2, sk, t, (in >> k) & 1u);
+            }
+        }
+        while (lanes_any(need != 0)) {
+            if (need) {
+                const int k = low_bit(need) - 8;
+                need &= need - 1;
+                const int ia = (k < 8) ? (int)((kTriS1 >> (4 * k)) & 15) : 8;
+                const int ib = (k < 8) ? (int)((kTriS2 >> (4 * k)) & 15) : k - 8;
+                const double sa = sh[ia * stride], sb = sh[ib * stride];
+                const SurfK &sk = t.surf[f.surf_at[k & 7]];
+                const EdgeK &e = (k < 8) ? sk.nest : t.edge[f.edge_at[k & 7]];
+                const bool closed = (k < 8) ? nest_closed(st, sa, sb, sk) : ((e.early != 0) & (sb > st));
+                if (!closed) edge_body(tn, sa, sb, e, t.F, (in >> (8 + k)) & 1u);
+            }
         }
     }
     return ((told > 0) ? 1.0 : -1.0) * tn;
+}
+
+// A direction's table into shared memory, by all `n` threads.
+__device__ __forceinline__ void copy_table(DirTable &dst, const DirTable &tab, int tid, int n)
+{
+    static_assert(sizeof(DirTable) % 16 == 0, "copied in 16-byte words");
+    for (int i = tid; i < (int)(sizeof(DirTable) / 16); i += n)
+        reinterpret_cast<int4 *>(&dst)[i] = reinterpret_cast<const int4 *>(&tab)[i];
+}
+
+// The same for one point with its sources named as in the reference
+// (:195-204); host code only (one point is not a warp).
+inline double point_update_fast(double told, double st, double xt, double yt, double xnt, double ynt, double txy,
+                                double txm, double tym, double txnyn, const DirTable *tab)
+{
+    const double s[9] = {xt, txy, yt, tym, xnt, txnyn, ynt, txm, st};
+    double sh[9];
+    float ch[9];
+    return point_update_fan(true, told, s, *tab, sh, ch, 1);
 }
 
 // ---------------------------------------------------------------------------

@@ -92,20 +92,11 @@ enum Variant {
     kVariantCompact = 2   // host-folded constants, solver calls compacted across the block
 };
 
-// WAVEFRONT tiles are 32 points along the plane's faster axis by
-// FOLD3D_WAVE_TV rows; one CTA of 32*FOLD3D_WAVE_TV threads works on a tile.
 // Pause between two polls of a dependency flag (ns; 0 polls back to back).
 #ifndef FOLD3D_POLL_NS
 #define FOLD3D_POLL_NS 32
 #endif
 constexpr unsigned kPollNs = FOLD3D_POLL_NS;
-
-// Single-solve dataflow passes over large planes: each warp owns whole items
-// (1), or the CTA's warps share each item's rows (0); build option.
-#ifndef FOLD3D_WAVE_WARP_ITEMS
-#define FOLD3D_WAVE_WARP_ITEMS 1
-#endif
-constexpr bool kWaveWarpItems = FOLD3D_WAVE_WARP_ITEMS != 0;
 
 // Items a batched pass's CTA claims at a time (1..32); build option.
 #ifndef FOLD3D_BATCH_CHUNK
@@ -114,19 +105,29 @@ constexpr bool kWaveWarpItems = FOLD3D_WAVE_WARP_ITEMS != 0;
 constexpr int kBatchChunk = FOLD3D_BATCH_CHUNK;
 static_assert(kBatchChunk >= 1 && kBatchChunk <= 32, "batch chunk");
 
+// Rows of the drift medium's tiles; build option, 0: by grid size
+// (drift_tile_rows in fold3d_api.cu).
+#ifndef FOLD3D_DRIFT_TV
+#define FOLD3D_DRIFT_TV 0
+#endif
+
+// WAVEFRONT tiles are 32 points along the plane's faster axis by some rows:
+// FOLD3D_WAVE_TV in single solves of the elliptical medium, where one CTA of
+// 32*FOLD3D_WAVE_TV threads works on a tile.
 #ifndef FOLD3D_WAVE_TV
 #define FOLD3D_WAVE_TV 4
 #endif
 constexpr int kWaveTV = FOLD3D_WAVE_TV;
 
-// Resident CTAs per SM the forward dataflow kernels are compiled for (their
-// register budget is 65536 / (32 * kWaveTV * this)); build options, each the
-// count that measured fastest with 32 x 4 tiles: drift 7 (512^3) and 7 on
-// planes of kLargePlaneTiles tiles or more (1280^3, warp-owned items; 8:
-// 2% slower, 6: 4% slower); the FP64 elliptical medium 6, and 7 on large
-// planes; the float32 one 8; batched solves (many small instances) 8.
+// Resident 128-thread CTAs per SM the forward dataflow kernels are compiled for
+// (their register budget is 65536 / (128 * this)); build options, each the
+// count that measured fastest.  Drift: 4 (128 registers; ms at 512^3, 8 sweeps,
+// and 1280^3, 2 sweeps, for 3, 4, 5 and 6: 342, 342, 333, 352 and 1269, 1126,
+// 1158, 1168): the update is one long chain per point, which spills and
+// reloads below 100 registers lengthen.  The FP64 elliptical medium 6, and 7 on
+// large planes; the float32 one 8; batched solves (many small instances) 8.
 #ifndef FOLD3D_WAVE_MINB_DRIFT
-#define FOLD3D_WAVE_MINB_DRIFT 7
+#define FOLD3D_WAVE_MINB_DRIFT 4
 #endif
 #ifndef FOLD3D_WAVE_MINB_ELLIP
 #define FOLD3D_WAVE_MINB_ELLIP 6
@@ -139,9 +140,6 @@ constexpr int kWaveTV = FOLD3D_WAVE_TV;
 #endif
 #ifndef FOLD3D_WAVE_MINB_LARGE
 #define FOLD3D_WAVE_MINB_LARGE 8  // large planes, float32 elliptical medium
-#endif
-#ifndef FOLD3D_WAVE_MINB_LARGE_DRIFT
-#define FOLD3D_WAVE_MINB_LARGE_DRIFT 7
 #endif
 #ifndef FOLD3D_WAVE_MINB_LARGE_ELLIP
 #define FOLD3D_WAVE_MINB_LARGE_ELLIP 7
@@ -156,13 +154,15 @@ static_assert(kWaveTV == 1 || kWaveTV == 2 || kWaveTV == 4 || kWaveTV == 8, "til
 struct WaveArgs {
     PlaneGeom pg;
     int nrm, ua, va, sg;         // normal axis, in-plane u / v axes, step direction
-    int ntu, ntv;                // 32 x kWaveTV tiles per plane (this orientation)
+    int ntu, ntv;                // tiles per plane (this orientation)
     int steps, first_src;        // plane steps of the pass and the first source plane
     unsigned epoch;              // number of this pass (monotonic per context)
     unsigned skip_from;          // passes numbered below this never skip
     unsigned long long timeout_ns;
     unsigned *flags;             // [steps][tiles]: pass number when the item finished
-    unsigned *mod[3];            // per orientation: [plane 0..n+1][tile]: last pass a point changed
+    // change maps, [plane 0..n+1][tile]: the last pass a point changed; of this
+    // pass's orientation, and of those with normal axes ua and va
+    unsigned *mod[3];
     int mod_ntu[3], mod_ntiles[3];
     unsigned *work;              // item counter (zeroed before each pass)
     unsigned *status;            // 0, or 1 after a wait gave up
@@ -206,13 +206,14 @@ constexpr unsigned kNoWinner = 0xffu;
 struct EllipDir;     // fold3d_ellip.cuh
 struct EllipParam;   // below, once EllipDir is complete
 
-// large: the variant compiled for passes over large planes (kLargePlaneTiles).
-cudaError_t launch_wave_pass(double *T, const WaveArgs &a, const DirTable &tab, int grid, cudaStream_t s,
-                             bool large = false);
-// The elliptical medium's field is double, or float when f32.
+// A pass of the drift medium over tiles of tv rows (1, 2, 4 or 8).
+cudaError_t launch_wave_pass(double *T, const WaveArgs &a, const DirTable &tab, int tv, int grid, cudaStream_t s);
+int drift_blocks_per_sm(int tv);
+// The elliptical medium's field is double, or float when f32.  large: the
+// variant compiled for passes over large planes (kLargePlaneTiles).
 cudaError_t launch_wave_pass_ellip(void *T, bool f32, const WaveArgs &a, const EllipParam &p, int grid, cudaStream_t s,
                                    bool large = false);
-int wave_blocks_per_sm(int medium, bool f32 = false, bool large = false);
+int wave_blocks_per_sm(bool f32, bool large);
 
 }  // namespace fold3d
 #include "fold3d_ellip.cuh"

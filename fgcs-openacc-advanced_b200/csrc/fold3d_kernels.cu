@@ -62,20 +62,29 @@ __global__ void __launch_bounds__(256) plane_kernel_fast(double *__restrict__ T,
                                                          const __grid_constant__ DirTable tab,
                                                          unsigned long long *__restrict__ maxd)
 {
+    __shared__ double s_fan[9][256];
+    __shared__ float s_dif[9][256];
+    __shared__ DirTable s_tab;
+    const int tid = threadIdx.x + 32 * threadIdx.y;
     const int u = blockIdx.x * 32 + threadIdx.x + 1;
     const int v = blockIdx.y * 8 + threadIdx.y + 1;
-    double delta = 0.0;
-    if (u <= g.nu && v <= g.nv) {
+    const bool active = u <= g.nu && v <= g.nv;
+    long long tgt = 0;
+    double told = 0.0, fan[9] = {};
+    if (active) {
         const long long src = src_off + (long long)u * g.su + (long long)v * g.sv;
-        const long long tgt = src + g.sn;
+        tgt = src + g.sn;
         const Nbr9 s = load_nbr(T, src, g);
-        const double told = T[tgt];
-        const double tnew =
-            point_update_fast(told, s.st, s.xt, s.yt, s.xnt, s.ynt, s.txy, s.txm, s.tym, s.txnyn, &tab);
-        T[tgt] = tnew;
-        delta = fabs(tnew - told);
+        const double got[9] = {s.xt, s.txy, s.yt, s.tym, s.xnt, s.txnyn, s.ynt, s.txm, s.st};
+#pragma unroll
+        for (int r = 0; r < 9; ++r) fan[r] = got[r];
+        told = T[tgt];
     }
-    if (maxd) block_max_to(delta, maxd);
+    copy_table(s_tab, tab, tid, 256);
+    __syncthreads();
+    const double tnew = point_update_fan(active, told, fan, s_tab, &s_fan[0][tid], &s_dif[0][tid], 256);
+    if (active) T[tgt] = tnew;
+    if (maxd) block_max_to(active ? fabs(tnew - told) : 0.0, maxd);
 }
 
 __global__ void __launch_bounds__(256) plane_kernel_literal(double *__restrict__ T, long long src_off,

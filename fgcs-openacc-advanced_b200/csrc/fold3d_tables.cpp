@@ -360,6 +360,75 @@ SurfK surf_consts(double F, double ax, double ay, double az, double hx, double h
     return k;
 }
 
+// x rounded down to float, a little further than one ulp.
+float float_below(double x) { return (float)(x - 1e-6 * std::fabs(x)); }
+
+// The float filter's constants (fold3d_fast.cuh, 5.) from the table's own.
+// The filter is on where its error bound holds: F^2 >= 1.1 |a|^2, spacings
+// within a factor of 8, and travel times of a cell far from float's range.
+EdgeF edge_filter(const EdgeK &k, double F)
+{
+    EdgeF f;
+    const double Fp = std::sqrt(k.g), ax = k.ax / Fp, az = k.az / Fp;
+    f.k = (float)(Fp / k.hx);
+    f.kz = (float)(Fp / k.hz);
+    f.ax = (float)ax;
+    f.az = (float)az;
+    f.ga = (float)(1.0 - az * az);
+    f.iga = (float)(1.0 / (1.0 - az * az));
+    f.fx = (float)(F * ax);
+    f.fz = (float)(F * az);
+    f.s1 = (float)(k.hz / (k.hx + k.hz));
+    f.s2 = (float)(k.hx / (k.hx + k.hz));
+    f.ka = (float)(1.0 + std::fabs(F * ax) + std::fabs(F * az));
+    f.K = k.fb_ok ? float_below(k.K) : HUGE_VALF;
+    return f;
+}
+
+void filter_table(const LocalFrameH &L, SideTable &t)
+{
+    SideFilter &f = t.flt;
+    const double F = t.F, az = t.az / F;
+    const double hmin = std::min(t.hz, std::min(L.hx, L.hy)), hmax = std::max(t.hz, std::max(L.hx, L.hy));
+    const bool scale = hmin / F > 1e-18 && hmax / F < 1e18 && F > 1e-9 && F < 1e9;
+    const bool on = scale && F * F >= 1.1 * (L.ax * L.ax + L.ay * L.ay + L.az * L.az) && hmax <= 8.0 * hmin;
+    f.every = scale ? 0u : 0xffffffu;
+    f.eps = on ? 1e-3f : HUGE_VALF;
+    f.faz = (float)az;
+    f.fg = (float)(1.0 - az * az);
+    f.fig = (float)(1.0 / (1.0 - az * az));
+    f.fkz = (float)(F / t.hz);
+    f.fhz = (float)(t.hz / F * (1.0 + 1e-6));
+    for (int k = 0; k < 8; ++k) {
+        const SurfK &s = t.surf[k];
+        TriF &q = f.tri[k];
+        q.kx = (float)(F / s.hx);
+        q.ky = (float)(F / s.hy);
+        q.ax = (float)(s.ax / F);
+        q.ay = (float)(s.ay / F);
+        q.r1 = (float)(s.hy / (s.hx + s.hy));
+        q.r2 = (float)(s.hx / (s.hx + s.hy));
+        q.s1 = (float)(t.hz / (s.hx + t.hz));
+        q.s2 = (float)(s.hx / (s.hx + t.hz));
+        f.ef[k] = edge_filter(s.nest, F);
+        f.ef[8 + k] = edge_filter(t.edge[k], F);
+        f.gB[k] = float_below(s.B);
+        f.gB[8 + k] = std::min(float_below(s.nest.B), f.ef[k].K);
+        f.gB[16 + k] = std::min(float_below(t.edge[k].B), f.ef[8 + k].K);
+    }
+    f.m_e1 = t.m_e1;
+    f.m_e2 = t.m_e2;
+    f.m_nest_early = t.m_nest_early;
+    f.m_edge_early = t.m_edge_early;
+    f.d1_ok = t.d1_ok;
+    f.K1 = t.K1;
+    f.named[0] = 0;
+    f.named[1] = 2;
+    for (int k = 0; k < 8; ++k) f.surf_at[k] = f.edge_at[k] = (unsigned char)k;
+    f.outer = f.gB[0];
+    for (int k = 1; k < 24; ++k) f.outer = std::min(f.outer, f.gB[k]);
+}
+
 void side_table(const LocalFrameH &L, bool negative, bool search, SideTable &t)
 {
     std::memset(&t, 0, sizeof t);
@@ -413,9 +482,53 @@ void side_table(const LocalFrameH &L, bool negative, bool search, SideTable &t)
         t.m_nest_early |= (unsigned)(t.surf[k].nest.early != 0) << k;
         t.m_edge_early |= (unsigned)(t.edge[k].early != 0) << k;
     }
+    filter_table(L, t);
 }
 
 }  // namespace
+
+void orient_table(DirTable &tab, bool x_is_u, int xs, int ys)
+{
+    static const int I[8] = {1, 1, 0, -1, -1, -1, 0, 1}, J[8] = {0, 1, 1, 1, 0, -1, -1, -1};
+    int at[8], tri[8];  // places of the local rim points and triangles
+    for (int r = 0; r < 8; ++r) {
+        const int du = x_is_u ? I[r] * xs : J[r] * ys, dv = x_is_u ? J[r] * ys : I[r] * xs;
+        at[r] = 0;
+        while (I[at[r]] != du || J[at[r]] != dv) ++at[r];
+    }
+    auto s1 = [](int k) { return (int)((kTriS1 >> (4 * k)) & 15u); };
+    auto s2 = [](int k) { return (int)((kTriS2 >> (4 * k)) & 15u); };
+    for (int k = 0; k < 8; ++k) {
+        tri[k] = 0;
+        while (s1(tri[k]) != at[s1(k)] || s2(tri[k]) != at[s2(k)]) ++tri[k];
+    }
+    auto bits = [](unsigned m, const int *to) {
+        unsigned r = 0;
+        for (int k = 0; k < 8; ++k) r |= ((m >> k) & 1u) << to[k];
+        return r;
+    };
+    for (SideTable &t : tab.side) {
+        const SideFilter a = t.flt;
+        SideFilter &f = t.flt;
+        for (int k = 0; k < 8; ++k) {
+            f.gB[tri[k]] = a.gB[k];
+            f.gB[8 + tri[k]] = a.gB[8 + k];
+            f.gB[16 + at[k]] = a.gB[16 + k];
+            f.tri[tri[k]] = a.tri[k];
+            f.ef[tri[k]] = a.ef[k];
+            f.ef[8 + at[k]] = a.ef[8 + k];
+            f.surf_at[tri[k]] = a.surf_at[k];
+            f.edge_at[at[k]] = a.edge_at[k];
+        }
+        f.m_e1 = bits(a.m_e1, tri);
+        f.m_e2 = bits(a.m_e2, tri);
+        f.m_nest_early = bits(a.m_nest_early, tri);
+        f.m_edge_early = bits(a.m_edge_early, at);
+        const int x = at[0], y = at[2];  // xt and yt
+        f.named[0] = (x & 3) == 0 ? x : y;
+        f.named[1] = (x & 3) == 0 ? y : x;
+    }
+}
 
 void build_dir_table(const LocalFrameH &L, DirTable &out, bool search)
 {

@@ -2,16 +2,18 @@
 // directional pass, tile dataflow between consecutive planes, and tiles
 // skipped when their inputs did not change.
 //
-// Work items are (plane step p, tile t) pairs of a pass, tiles being
-// 32 x kWaveTV points of a plane, numbered plane-major.  Every CTA claims the next item
-// from an atomic counter.  Item (p, t) reads the source plane written by
+// Work items are (plane step p, tile t) pairs of a pass, tiles being 32 points
+// by a few rows of a plane, numbered plane-major.  A worker -- a warp in the
+// drift medium's passes, a CTA in the elliptical medium's -- claims the next
+// item from an atomic counter.  Item (p, t) reads the source plane written by
 // step p-1 only within t's 1-point halo, i.e. from the 3 x 3 tiles around t,
 // so it waits for exactly those items (their completion flags), not for the
 // whole previous plane: consecutive planes overlap and no plane-wide barrier
-// or launch separates them.  Items are claimed in increasing order, so every
-// item an item waits for is held by a CTA that is already running; the
-// waits always end.  They are bounded anyway: after a time limit the CTA
-// raises the status word and every CTA leaves (FOLD3D_ERR_TIMEOUT).
+// or launch separates them.  Items are claimed in increasing order and a worker
+// processes its claims in order, so the lowest unfinished item is always held
+// by a running worker that is at it; the waits always end.  They are bounded
+// anyway: after a time limit the worker raises the status word and every
+// worker leaves (FOLD3D_ERR_TIMEOUT).
 //
 // Skipping.  A point update is min(T_old, M(nine source values, side)) (see
 // fold3d_fast.cuh), so re-evaluating a tile whose source neighbourhood has
@@ -29,13 +31,12 @@
 // step p-1 of the current pass changed the source plane comes with its
 // completion flags, which hold (pass << 1) | changed.
 //
-// Synchronisation: a CTA publishes an item with __syncthreads and a
-// gpu-scope release store into the item's flag; in a waiting CTA, nine
-// threads poll the nine neighbour flags in parallel with acquire loads and
-// then release the block with __syncthreads.  Each CTA claims its next item
-// while it works on the current one.  Field values written inside the launch are read with
-// L2-cached loads (ld.global.cg), never through the non-coherent read-only
-// path.
+// Synchronisation: an item is published with a barrier of its worker's threads
+// (__syncwarp or __syncthreads) and a gpu-scope release of the item's flag; nine
+// lanes of the waiting worker poll the nine neighbour flags in parallel with
+// acquire loads before a barrier.  Field values written inside the launch are
+// read with L2-cached loads (ld.global.cg), never through the non-coherent
+// read-only path.
 #include <cstring>
 
 #include "fold3d_ellip.cuh"
@@ -56,15 +57,13 @@ __device__ __forceinline__ bool bits_differ(float a, float b) { return __float_a
 
 }  // namespace
 
-constexpr int kWaveThreads = 32 * kWaveTV;
+constexpr int kWaveThreads = 128;  // four warps
+
 
 template <int MED, class R, bool LARGE> constexpr int wave_min_blocks()
 {
-    return LARGE ? (MED == kMediumDrift   ? FOLD3D_WAVE_MINB_LARGE_DRIFT
-                    : sizeof(R) == 8      ? FOLD3D_WAVE_MINB_LARGE_ELLIP
-                                          : FOLD3D_WAVE_MINB_LARGE)
-                 : MED == kMediumDrift ? FOLD3D_WAVE_MINB_DRIFT
-                                       : (sizeof(R) == 8 ? FOLD3D_WAVE_MINB_ELLIP : FOLD3D_WAVE_MINB_ELLIP_F32);
+    return LARGE ? (sizeof(R) == 8 ? FOLD3D_WAVE_MINB_LARGE_ELLIP : FOLD3D_WAVE_MINB_LARGE)
+                 : (sizeof(R) == 8 ? FOLD3D_WAVE_MINB_ELLIP : FOLD3D_WAVE_MINB_ELLIP_F32);
 }
 
 // Medium-dependent launch parameters: the drift medium's constant table, or
@@ -77,6 +76,58 @@ template <> struct WaveMedium<kMediumEllip> {
     using type = EllipParam;
 };
 
+// A lane's point (u, v) of the target plane src + sg: update it from the source
+// plane and store it; whether it changed.
+template <class R>
+__device__ __forceinline__ bool ellip_point(R *__restrict__ T, const WaveArgs &a, const EllipParam &tab, int src, int u,
+                                            int v, double &dmax, unsigned &evaluated)
+{
+    const PlaneGeom &g = a.pg;
+    if (u > g.nu || v > g.nv) return false;
+    const long long s = (long long)src * g.s_nrm + (long long)u * g.su + (long long)v * g.sv, d = s + g.sn;
+    const R told = ld_cg(T + d), st = fabs(ld_cg(T + s));
+    R nb[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) nb[r] = fabs(ld_cg(T + s + ell_ri(r) * g.sx + ell_rj(r) * g.sy));
+    int win;
+    const R tnew = point_update_ellip(told, st, nb, ell_local<R>(tab.med, tab.dir, d), win);
+    ++evaluated;
+    if (!bits_differ(tnew, told)) return false;
+    if (a.winners) a.winners[d] = (win < 0) ? (unsigned char)kNoWinner : (unsigned char)(a.dir * kEllipCands + win);
+    T[d] = tnew;
+    dmax = fmax(dmax, (double)fabs(tnew - told));
+    return true;
+}
+
+// Marks the tile of changed point (u, v) of plane tgt in an in-plane
+// orientation: Q = 1, planes u of normal axis ua; Q = 2, planes v of va.
+template <int Q, int TV>
+__device__ __forceinline__ void wave_mark(const WaveArgs &a, int u, int v, int tgt)
+{
+    const int other = (Q == 1) ? v : u;
+    const bool first = a.nrm < ((Q == 1) ? a.va : a.ua);  // the pass's normal is that orientation's faster axis
+    const int cu = first ? tgt : other, cv = first ? other : tgt;
+    a.mod[Q][(long long)(Q == 1 ? u : v) * a.mod_ntiles[Q] + ((cv - 1) / TV) * a.mod_ntu[Q] + ((cu - 1) >> 5)] = a.epoch;
+}
+
+// x / n and the remainder r for 0 <= x, n > 0; inv = 1/n rounded.  The product
+// is off by at most one for quotients below 2^22, and corrected from the
+// remainder (in as many steps as it takes beyond that).
+__device__ __forceinline__ int wave_div(int x, int n, float inv, int &r)
+{
+    int q = (int)((float)x * inv);
+    r = x - q * n;
+    while (r < 0) {
+        --q;
+        r += n;
+    }
+    while (r >= n) {
+        ++q;
+        r -= n;
+    }
+    return q;
+}
+
 // One work item (step p, tile t) of one grid, for all threads of the CTA:
 // wait for the 3 x 3 tiles of step p-1, then skip or update the tile, then
 // publish its flag.  Adds each changed point's |dT| into dmax and the
@@ -85,7 +136,7 @@ template <> struct WaveMedium<kMediumEllip> {
 template <int MED, class R, int TV = kWaveTV>
 __device__ __forceinline__ bool wave_item(R *__restrict__ T, const WaveArgs &a,
                                           const typename WaveMedium<MED>::type &tab, int item, double &dmax,
-                                          unsigned long long &evaluated)
+                                          unsigned &evaluated)
 {
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
@@ -106,21 +157,11 @@ __device__ __forceinline__ bool wave_item(R *__restrict__ T, const WaveArgs &a,
         const int nu = tu + tid % 3 - 1, nv = tv + tid / 3 - 1;
         if (nu >= 0 && nu < a.ntu && nv >= 0 && nv < a.ntv) {
             const int nt = nv * a.ntu + nu;
-            if (may_skip) recent = (__ldcg(a.mod[a.nrm] + (long long)src * ntiles + nt) + 5u >= a.epoch);
+            if (may_skip) recent = (__ldcg(a.mod[0] + (long long)src * ntiles + nt) + 5u >= a.epoch);
             if (p > 0) {
-                const unsigned *fl = a.flags + (long long)(p - 1) * ntiles + nt;
-                const unsigned long long t0 = global_ns();
-                unsigned spins = 0, f;
-                while ((f = ld_acquire(fl)) < want) {
-                    if (++spins > (1u << 26) || global_ns() - t0 > a.timeout_ns ||
-                        *(volatile unsigned *)a.status != 0) {
-                        atomicCAS(a.status, 0u, 1u);  // FOLD3D_ERR_TIMEOUT
-                        timed_out = 1;
-                        break;
-                    }
-                    if (kPollNs) __nanosleep(kPollNs);
-                }
-                if (!timed_out) recent |= (int)(f & 1u);
+                const unsigned f = wait_flag(a.flags + (long long)(p - 1) * ntiles + nt, want, a.status, a.timeout_ns);
+                timed_out = f == 0;
+                recent |= (int)(f & 1u);
             }
         }
     }
@@ -131,50 +172,13 @@ __device__ __forceinline__ bool wave_item(R *__restrict__ T, const WaveArgs &a,
     if (!skip) {
         const int u = tu * 32 + lane + 1;
         const int v = tv * TV + warp + 1;
-        if (u <= g.nu && v <= g.nv) {
-            const long long s = (long long)src * g.s_nrm + (long long)u * g.su + (long long)v * g.sv;
-            const long long d = s + g.sn;
-            const R st = fabs(ld_cg(T + s));
-            const R xt = fabs(ld_cg(T + s + g.sx));
-            const R yt = fabs(ld_cg(T + s + g.sy));
-            const R xnt = fabs(ld_cg(T + s - g.sx));
-            const R ynt = fabs(ld_cg(T + s - g.sy));
-            const R txm = fabs(ld_cg(T + s + g.sx - g.sy));
-            const R txy = fabs(ld_cg(T + s + g.sx + g.sy));
-            const R tym = fabs(ld_cg(T + s - g.sx + g.sy));
-            const R txnyn = fabs(ld_cg(T + s - g.sx - g.sy));
-            const R told = ld_cg(T + d);
-            R tnew;
-            if constexpr (MED == kMediumDrift) {
-                static_assert(sizeof(R) == 8, "the drift medium is solved in double");
-                tnew = point_update_fast(told, st, xt, yt, xnt, ynt, txy, txm, tym, txnyn, &tab);
-            } else {
-                const R nb[8] = {xt, txy, yt, tym, xnt, txnyn, ynt, txm};
-                int win;
-                tnew = point_update_ellip(told, st, nb, ell_local<R>(tab.med, tab.dir, d), win);
-                if (a.winners && bits_differ(tnew, told))
-                    a.winners[d] = (win < 0) ? (unsigned char)kNoWinner : (unsigned char)(a.dir * kEllipCands + win);
-            }
-            if (bits_differ(tnew, told)) {
-                T[d] = tnew;
-                changed = 1;
-                dmax = fmax(dmax, (double)fabs(tnew - told));
-                // mark the point's tile in the two other orientations
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    const int b = (q == 0) ? a.ua : a.va;
-                    const int ub = (b == 0) ? 1 : 0, vb = (b == 2) ? 1 : 2;
-                    const int cb = (q == 0) ? u : v;
-                    const int cu = (ub == a.nrm) ? tgt : (ub == a.ua) ? u : v;
-                    const int cv = (vb == a.nrm) ? tgt : (vb == a.ua) ? u : v;
-                    const int tile = ((cv - 1) / TV) * a.mod_ntu[b] + ((cu - 1) >> 5);
-                    a.mod[b][(long long)cb * a.mod_ntiles[b] + tile] = a.epoch;
-                }
-            }
-            ++evaluated;
+        if (ellip_point<R>(T, a, tab, src, u, v, dmax, evaluated)) {
+            changed = 1;
+            wave_mark<1, TV>(a, u, v, tgt);
+            wave_mark<2, TV>(a, u, v, tgt);
         }
         changed = __syncthreads_or(changed);
-        if (changed && tid == 0) a.mod[a.nrm][(long long)tgt * ntiles + t] = a.epoch;
+        if (changed && tid == 0) a.mod[0][(long long)tgt * ntiles + t] = a.epoch;
     }
     // publish: the barrier makes every thread's stores precede thread 0's
     // release store, which orders them (cumulatively) before the flag
@@ -183,109 +187,8 @@ __device__ __forceinline__ bool wave_item(R *__restrict__ T, const WaveArgs &a,
     return true;
 }
 
-// The same work item done by one warp alone: its 32 lanes take the tile's
-// rows one after the other, lanes 0..8 watch the nine neighbour flags, and
-// lane 0 publishes after a __syncwarp (which orders every lane's stores
-// before lane 0's release store).  The warps of a CTA each own their items,
-// so none waits at a CTA barrier for the slowest row of another's.
-template <int MED, class R, int TV = kWaveTV>
-__device__ __forceinline__ bool wave_item_warp(R *__restrict__ T, const WaveArgs &a,
-                                               const typename WaveMedium<MED>::type &tab, int item, double &dmax,
-                                               unsigned long long &evaluated)
-{
-    const int lane = threadIdx.x & 31;
-    const PlaneGeom &g = a.pg;
-    const int ntiles = a.ntu * a.ntv;
-    const unsigned want = a.epoch << 1;  // flags hold (pass << 1) | changed
-    const bool may_skip = a.epoch >= a.skip_from;
-    const int p = item / ntiles, t = item - p * ntiles;
-    const int tu = t % a.ntu, tv = t / a.ntu;
-    const int src = a.first_src + p * a.sg;
-    const int tgt = src + a.sg;
-
-    int timed_out = 0, recent = 0;
-    if (lane < 9) {
-        const int nu = tu + lane % 3 - 1, nv = tv + lane / 3 - 1;
-        if (nu >= 0 && nu < a.ntu && nv >= 0 && nv < a.ntv) {
-            const int nt = nv * a.ntu + nu;
-            if (may_skip) recent = (__ldcg(a.mod[a.nrm] + (long long)src * ntiles + nt) + 5u >= a.epoch);
-            if (p > 0) {
-                const unsigned *fl = a.flags + (long long)(p - 1) * ntiles + nt;
-                const unsigned long long t0 = global_ns();
-                unsigned spins = 0, f;
-                while ((f = ld_acquire(fl)) < want) {
-                    if (++spins > (1u << 26) || global_ns() - t0 > a.timeout_ns ||
-                        *(volatile unsigned *)a.status != 0) {
-                        atomicCAS(a.status, 0u, 1u);  // FOLD3D_ERR_TIMEOUT
-                        timed_out = 1;
-                        break;
-                    }
-                    if (kPollNs) __nanosleep(kPollNs);
-                }
-                if (!timed_out) recent |= (int)(f & 1u);
-            }
-        }
-    }
-    if (__any_sync(0xffffffffu, timed_out)) return false;
-    const bool skip = may_skip && !__any_sync(0xffffffffu, recent);
-
-    int changed = 0;
-    if (!skip) {
-        const int u = tu * 32 + lane + 1;
-        for (int r = 0; r < TV; ++r) {
-            const int v = tv * TV + r + 1;
-            if (u <= g.nu && v <= g.nv) {
-                const long long s = (long long)src * g.s_nrm + (long long)u * g.su + (long long)v * g.sv;
-                const long long d = s + g.sn;
-                const R st = fabs(ld_cg(T + s));
-                const R xt = fabs(ld_cg(T + s + g.sx));
-                const R yt = fabs(ld_cg(T + s + g.sy));
-                const R xnt = fabs(ld_cg(T + s - g.sx));
-                const R ynt = fabs(ld_cg(T + s - g.sy));
-                const R txm = fabs(ld_cg(T + s + g.sx - g.sy));
-                const R txy = fabs(ld_cg(T + s + g.sx + g.sy));
-                const R tym = fabs(ld_cg(T + s - g.sx + g.sy));
-                const R txnyn = fabs(ld_cg(T + s - g.sx - g.sy));
-                const R told = ld_cg(T + d);
-                R tnew;
-                if constexpr (MED == kMediumDrift) {
-                    tnew = point_update_fast(told, st, xt, yt, xnt, ynt, txy, txm, tym, txnyn, &tab);
-                } else {
-                    const R nb[8] = {xt, txy, yt, tym, xnt, txnyn, ynt, txm};
-                    int win;
-                    tnew = point_update_ellip(told, st, nb, ell_local<R>(tab.med, tab.dir, d), win);
-                    if (a.winners && bits_differ(tnew, told))
-                        a.winners[d] =
-                            (win < 0) ? (unsigned char)kNoWinner : (unsigned char)(a.dir * kEllipCands + win);
-                }
-                if (bits_differ(tnew, told)) {
-                    T[d] = tnew;
-                    changed = 1;
-                    dmax = fmax(dmax, (double)fabs(tnew - told));
-#pragma unroll
-                    for (int q = 0; q < 2; ++q) {  // the point's tile in the two other orientations
-                        const int b = (q == 0) ? a.ua : a.va;
-                        const int ub = (b == 0) ? 1 : 0, vb = (b == 2) ? 1 : 2;
-                        const int cb = (q == 0) ? u : v;
-                        const int cu = (ub == a.nrm) ? tgt : (ub == a.ua) ? u : v;
-                        const int cv = (vb == a.nrm) ? tgt : (vb == a.ua) ? u : v;
-                        const int tile = ((cv - 1) / TV) * a.mod_ntu[b] + ((cu - 1) >> 5);
-                        a.mod[b][(long long)cb * a.mod_ntiles[b] + tile] = a.epoch;
-                    }
-                }
-                ++evaluated;
-            }
-        }
-        changed = __any_sync(0xffffffffu, changed);
-        if (changed && lane == 0) a.mod[a.nrm][(long long)tgt * ntiles + t] = a.epoch;
-    }
-    __syncwarp();
-    if (lane == 0) st_release(a.flags + item, want | (unsigned)changed);
-    return true;
-}
-
 // Block-wide maximum of d into *out (IEEE bits) and sum of e into *sum.
-template <int TV = kWaveTV>
+template <int TV>
 __device__ __forceinline__ void wave_flush(double d, unsigned long long e, unsigned long long *out,
                                            unsigned long long *sum)
 {
@@ -308,6 +211,139 @@ __device__ __forceinline__ void wave_flush(double d, unsigned long long e, unsig
     __syncthreads();
 }
 
+// A pass of the drift medium.  Every warp claims and processes whole items
+// of 32 x TV points on its own, the tile's rows one after another, and
+// publishes them with one fence; no warp waits at a CTA barrier for another's
+// rows.  A row's nine source values are the last row's shifted by one, with
+// three new ones read while the last row is worked on.
+//
+// What bounds it: the latency of a point's update and of the exchange between
+// plane steps, not bytes (10 DRAM bytes per update) and not issue (47% of the
+// cycles at 1280^2 planes).  Per row of 32 points it runs 520 warp instructions
+// (about 930 before the float filter).  In a settled field (no tile skipped)
+// a plane step takes 6.6, 9.6, 12.6 and 61 us at 64, 256, 512 and 1280 points
+// per axis, of which the claims, waits and publishing alone 2.5, 4.0, 5.7 and 9.
+// ms before (a CTA per 32 x 4 tile, FP64 gates) and now: 64^3, 8 sweeps 36 ->
+// 20; 512^3, 8 sweeps 455 -> 335; 1280^3, 2 sweeps 1515 -> 1126.
+template <int TV>
+__global__ void __launch_bounds__(kWaveThreads, FOLD3D_WAVE_MINB_DRIFT)
+    drift_pass_kernel(double *__restrict__ T, WaveArgs a, const __grid_constant__ DirTable tab)
+{
+    __shared__ DirTable s_tab;
+    __shared__ double s_fan[9 * kWaveThreads];
+    __shared__ float s_dif[9 * kWaveThreads];
+    copy_table(s_tab, tab, threadIdx.x, kWaveThreads);
+    __syncthreads();
+    const PlaneGeom &g = a.pg;
+    const int lane = threadIdx.x & 31;
+    const int ntiles = a.ntu * a.ntv;
+    const unsigned total = (unsigned)(a.steps * ntiles);
+    const float inv_tiles = 1.0f / (float)ntiles, inv_ntu = 1.0f / (float)a.ntu;
+    const unsigned want = a.epoch << 1;  // flags hold (pass << 1) | changed
+    const bool may_skip = a.epoch >= a.skip_from;
+    double dmax = 0.0;
+    unsigned evaluated = 0;
+    // Lanes 0..8 each watch one tile of an item's 3 x 3 neighbourhood: its
+    // change mark from earlier passes, and its step p-1 flag (which also says
+    // whether that item changed the source plane).  watch() gives the lane's
+    // flag, or NULL where there is nothing to wait for.
+    auto watch = [&](unsigned item, int &p, int &t, int &tu, int &tv, bool &recent) -> const unsigned * {
+        p = wave_div((int)item, ntiles, inv_tiles, t);
+        tv = wave_div(t, a.ntu, inv_ntu, tu);
+        const int nu = tu + lane % 3 - 1, nv = tv + lane / 3 - 1, nt = nv * a.ntu + nu;
+        const bool in = lane < 9 && nu >= 0 && nu < a.ntu && nv >= 0 && nv < a.ntv;
+        recent = in && may_skip && __ldcg(a.mod[0] + (long long)(a.first_src + p * a.sg) * ntiles + nt) + 5u >= a.epoch;
+        return (in && p > 0) ? a.flags + (long long)(p - 1) * ntiles + nt : nullptr;
+    };
+    // The warp holds two claimed items: the flags of the second are read while
+    // the first is worked on, and the fence that publishes the first also
+    // orders that read before the second's loads.
+    unsigned ahead = 0;
+    if (lane == 0) ahead = atomicAdd(a.work, 1u);
+    unsigned item = __shfl_sync(0xffffffffu, ahead, 0);
+    if (lane == 0) ahead = atomicAdd(a.work, 1u);
+    int p = 0, t = 0, tu = 0, tv = 0;
+    bool recent = false;
+    const unsigned *fl = item < total ? watch(item, p, t, tu, tv, recent) : nullptr;
+    unsigned f = 0;
+    while (item < total) {
+        bool gave_up = false;
+        if (fl && f < want) {
+            f = wait_flag(fl, want, a.status, a.timeout_ns);
+            gave_up = f == 0;
+        }
+        recent |= fl && (f & 1u);
+        if (__any_sync(0xffffffffu, gave_up)) break;
+        const bool skip = may_skip && !__any_sync(0xffffffffu, recent);
+        const unsigned next = __shfl_sync(0xffffffffu, ahead, 0);
+        if (lane == 0) ahead = atomicAdd(a.work, 1u);
+        const int src = a.first_src + p * a.sg, tgt = src + a.sg, u = tu * 32 + lane + 1, v0 = tv * TV + 1;
+        const int t0 = t, last = min(TV, g.nv - v0 + 1);
+        const double *s = T + ((long long)src * g.s_nrm + (long long)u * g.su + (long long)v0 * g.sv);
+        const bool active = u <= g.nu && !skip;
+        // source rows v0 - 1 .. v0 + 1, and the target
+        double w[3][3] = {}, told = 0.0;
+        if (active) {
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) w[i][j] = fabs(ld_cg(s + (i - 1) * g.sv + (j - 1) * g.su));
+            told = ld_cg(s + g.sn);
+        }
+        if (next < total) {
+            fl = watch(next, p, t, tu, tv, recent);
+            f = fl ? ld_relaxed(fl) : 0u;
+        }
+        unsigned any = 0;
+        if (!skip) {
+#pragma unroll 1
+            for (int r = 0; r < last; ++r, s += g.sv) {
+                double w3[3] = {}, told3 = 0.0;  // the next row's new sources and target
+                if (TV > 1 && active && r + 1 < last) {
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) w3[j] = fabs(ld_cg(s + 2 * g.sv + (j - 1) * g.su));
+                    told3 = ld_cg(s + g.sv + g.sn);
+                }
+                const double fan[9] = {w[1][2], w[2][2], w[2][1], w[2][0], w[1][0], w[0][0], w[0][1], w[0][2], w[1][1]};
+                const double tnew =
+                    point_update_fan(active, told, fan, s_tab, &s_fan[threadIdx.x], &s_dif[threadIdx.x], kWaveThreads);
+                const bool changed = active && bits_differ(tnew, told);
+                evaluated += active;
+                if (changed) {
+                    const_cast<double *>(s)[g.sn] = tnew;
+                    dmax = fmax(dmax, fabs(tnew - told));
+                    wave_mark<2, TV>(a, u, v0 + r, tgt);
+                }
+                any |= (unsigned)changed;
+                if (TV > 1) {
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) {
+                        w[0][j] = w[1][j];
+                        w[1][j] = w[2][j];
+                        w[2][j] = w3[j];
+                    }
+                    told = told3;
+                }
+            }
+            if (any) wave_mark<1, TV>(a, u, v0, tgt);
+            any = __any_sync(0xffffffffu, any);
+        }
+        __syncwarp();
+        fence_acq_rel();
+        if (lane == 0) {
+            st_relaxed(a.flags + item, want | any);
+            if (any) a.mod[0][(long long)tgt * ntiles + t0] = a.epoch;
+        }
+        __syncwarp();
+        item = next;
+    }
+    __syncthreads();
+    wave_flush<kWaveThreads / 32>(dmax, evaluated, a.maxd, a.evaluated);
+}
+
+// A pass of the elliptical medium: the warps of a CTA share each item's rows.
+// (Its point update is long straight-line code; warps that run it together
+// fetch it together.)
 template <int MED, class R, bool LARGE>
 __global__ void __launch_bounds__(kWaveThreads, (wave_min_blocks<MED, R, LARGE>()))
     wave_pass_kernel(R *__restrict__ T, WaveArgs a, const __grid_constant__ typename WaveMedium<MED>::type tab)
@@ -315,35 +351,7 @@ __global__ void __launch_bounds__(kWaveThreads, (wave_min_blocks<MED, R, LARGE>(
     __shared__ int s_next;
     const long long total = (long long)a.steps * a.ntu * a.ntv;
     double dmax = 0.0;
-    unsigned long long evaluated = 0;
-    if constexpr (kWaveWarpItems && LARGE && MED == kMediumDrift) {
-        // drift medium, large planes: every warp claims and processes its own
-        // items (wave_item_warp).  A plane then has enough tiles to keep all
-        // warps busy, and no warp waits at a CTA barrier for another's row.
-        // On smaller planes the plane-to-plane chain binds instead, and an
-        // item shared by the CTA's warps (each one row) finishes sooner; the
-        // elliptical medium's larger per-point state made warp items slower
-        // on large planes too (measured).
-        const int lane = threadIdx.x & 31;
-        int item = -1;
-        if (lane == 0) {
-            const unsigned w = atomicAdd(a.work, 1u);
-            item = (w < total) ? (int)w : -1;
-        }
-        item = __shfl_sync(0xffffffffu, item, 0);
-        while (item >= 0) {
-            int next = -1;  // claimed now, processed after this one
-            if (lane == 0 && *(volatile unsigned *)a.status == 0) {
-                const unsigned w = atomicAdd(a.work, 1u);
-                if (w < total) next = (int)w;
-            }
-            next = __shfl_sync(0xffffffffu, next, 0);
-            if (!wave_item_warp<MED, R>(T, a, tab, item, dmax, evaluated)) break;
-            item = next;
-        }
-        wave_flush(dmax, evaluated, a.maxd, a.evaluated);
-        return;
-    }
+    unsigned evaluated = 0;
     if (threadIdx.x == 0) {
         const unsigned w = atomicAdd(a.work, 1u);
         s_next = (w < total) ? (int)w : -1;
@@ -354,16 +362,12 @@ __global__ void __launch_bounds__(kWaveThreads, (wave_min_blocks<MED, R, LARGE>(
         if (item < 0) break;
         __syncthreads();  // every thread has read s_next
         if (threadIdx.x == 0) {  // claim the next item now; it is processed after this one
-            int it = -1;
-            if (*(volatile unsigned *)a.status == 0) {
-                const unsigned w = atomicAdd(a.work, 1u);
-                if (w < total) it = (int)w;
-            }
-            s_next = it;
+            const unsigned w = atomicAdd(a.work, 1u);
+            s_next = (w < total) ? (int)w : -1;
         }
-        if (!wave_item<MED, R>(T, a, tab, item, dmax, evaluated)) break;
+        if (!wave_item<MED, R, kWaveTV>(T, a, tab, item, dmax, evaluated)) break;
     }
-    wave_flush(dmax, evaluated, a.maxd, a.evaluated);
+    wave_flush<kWaveTV>(dmax, evaluated, a.maxd, a.evaluated);
 }
 
 // ---------------------------------------------------------------------------
@@ -405,7 +409,7 @@ __global__ void __launch_bounds__(32 * TV, batch_min_blocks<TV>()) batch_pass_ke
     // The instance stays staged, and its largest change and evaluated points
     // are flushed only when the CTA moves to another one.
     double dmax = 0.0;
-    unsigned long long evaluated = 0;
+    unsigned evaluated = 0;
     for (int q = 0;; ++q) {
         if (q == s_n) {  // the same for every thread
             const int c0 = s_next;
@@ -417,12 +421,8 @@ __global__ void __launch_bounds__(32 * TV, batch_min_blocks<TV>()) batch_pass_ke
                     batch_locate(b.step_off, b.step_k, b.tile_pre, b.max_steps, c0 + (int)threadIdx.x,
                                  s_loc[threadIdx.x][0], s_loc[threadIdx.x][1]);
                 if (threadIdx.x == 0) {
-                    int it = -1;
-                    if (*(volatile unsigned *)b.status == 0) {
-                        const unsigned w = atomicAdd(b.work, (unsigned)kBatchChunk);
-                        if (w < total) it = (int)w;
-                    }
-                    s_next = it;
+                    const unsigned w = atomicAdd(b.work, (unsigned)kBatchChunk);
+                    s_next = (w < total) ? (int)w : -1;
                     s_n = n;
                 }
             }
@@ -539,10 +539,15 @@ int batch_blocks_per_sm(bool f32, int tv)
     return tv == 2 ? batch_occupancy<2>(f32) : tv == 8 ? batch_occupancy<8>(f32) : batch_occupancy<4>(f32);
 }
 
-cudaError_t launch_wave_pass(double *T, const WaveArgs &a, const DirTable &tab, int grid, cudaStream_t s, bool large)
+cudaError_t launch_wave_pass(double *T, const WaveArgs &a, const DirTable &tab, int tv, int grid, cudaStream_t s)
 {
-    if (large) wave_pass_kernel<kMediumDrift, double, true><<<grid, kWaveThreads, 0, s>>>(T, a, tab);
-    else wave_pass_kernel<kMediumDrift, double, false><<<grid, kWaveThreads, 0, s>>>(T, a, tab);
+    switch (tv) {
+    case 1: drift_pass_kernel<1><<<grid, kWaveThreads, 0, s>>>(T, a, tab); break;
+    case 2: drift_pass_kernel<2><<<grid, kWaveThreads, 0, s>>>(T, a, tab); break;
+    case 4: drift_pass_kernel<4><<<grid, kWaveThreads, 0, s>>>(T, a, tab); break;
+    case 8: drift_pass_kernel<8><<<grid, kWaveThreads, 0, s>>>(T, a, tab); break;
+    default: return cudaErrorInvalidValue;
+    }
     return cudaGetLastError();
 }
 
@@ -568,16 +573,19 @@ template <class K> static int occupancy(K kernel)
     return n > 0 ? n : 1;
 }
 
-int wave_blocks_per_sm(int medium, bool f32, bool large)
+int wave_blocks_per_sm(bool f32, bool large)
 {
-    if (medium != kMediumEllip)
-        return large ? occupancy(wave_pass_kernel<kMediumDrift, double, true>)
-                     : occupancy(wave_pass_kernel<kMediumDrift, double, false>);
     if (f32)
         return large ? occupancy(wave_pass_kernel<kMediumEllip, float, true>)
                      : occupancy(wave_pass_kernel<kMediumEllip, float, false>);
     return large ? occupancy(wave_pass_kernel<kMediumEllip, double, true>)
                  : occupancy(wave_pass_kernel<kMediumEllip, double, false>);
+}
+
+int drift_blocks_per_sm(int tv)
+{
+    return tv == 1 ? occupancy(drift_pass_kernel<1>) : tv == 2 ? occupancy(drift_pass_kernel<2>)
+         : tv == 8 ? occupancy(drift_pass_kernel<8>) : occupancy(drift_pass_kernel<4>);
 }
 
 }  // namespace fold3d
