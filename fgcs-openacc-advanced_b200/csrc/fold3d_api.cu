@@ -182,7 +182,7 @@ struct fold3d_ctx {
     double *tune_T = nullptr;                // autotuner: copies of a few instances' fields
     size_t tune_cells = 0;
     int wave_bps[2][2] = {};                 // [f32][large plane] resident CTAs per SM, elliptical medium
-    int drift_bps[9] = {};                   // and drift medium, by tile rows
+    int drift_bps[5] = {};                   // and drift medium, by tile rows
     // batched solves: per-instance scratch and per-direction staging
     std::vector<int> bkey;                   // dims of the instances the scratch is sized for
     unsigned *b_scratch = nullptr;           // flags and change maps of all instances
@@ -488,7 +488,6 @@ static EllipParam ellip_param(const fold3d_grid &g, const EllipMedium &m, int di
     return p;
 }
 
-// T: double, or float when f32 (elliptical medium only).
 // Rows of the drift medium's tiles, from the mean number of 32-point rows in a
 // plane step.  An item's rows run one after another on one warp, so few rows
 // per item keep the plane-to-plane chain short, and many share the cost of a
@@ -503,6 +502,7 @@ static int drift_tile_rows(const fold3d_grid &g)
     return rows < 12000.0 ? 1 : rows < 32000.0 ? 2 : 4;
 }
 
+// T: double, or float when f32 (elliptical medium only).
 static int solve_wavefront(fold3d_ctx *c, const fold3d_grid &g, const fold3d_medium *fm, const EllipMedium *em,
                            void *T, bool f32, const fold3d_opts &o, cudaStream_t s, fold3d_report *rep,
                            unsigned char *winners = nullptr)

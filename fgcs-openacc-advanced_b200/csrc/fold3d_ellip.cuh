@@ -304,6 +304,438 @@ __host__ __device__ __forceinline__ R point_update_ellip(R told, R st, const R n
     }
     return ((told > R(0)) ? R(1) : R(-1)) * tn;
 }
+// ---------------------------------------------------------------------------
+// The FP64 update with a float filter.
+//
+// Over one triangle of the fan, f(p) = t(p) + ||X - p||_M is convex, and its
+// smallest value there is at its stationary point u over the whole plane when
+// u lies inside, and otherwise on an edge that u lies beyond (walking from the
+// smallest point towards u lowers f, so the walk leaves the triangle at once).
+// In the scaled local frame, with P the in-plane part of A, p0 = P^-1 (xz, yz)
+// the foot of X, r = ||X - p0||^2 and g the gradient of t on the triangle,
+// h = P^-1 g and s = g.h, u = p0 - n h with n = sqrt(r / (1 - s)) and
+// f(u) = t(p0) + sqrt(r (1 - s)).  For s >= 1 there is no such u, but any point
+// far enough along -h has a lower f than the triangle and serves as well.  P,
+// p0 and r are the same for all eight triangles.
+//
+// The filter works this out in float for the triangles that could hold a time
+// below the current one, from differences rounded once, and keeps a candidate
+// only where the smallest value over the fan can lie at it: a triangle's
+// interior when u may be inside; a spoke when u may lie beyond it seen from
+// both its triangles, a rim edge from its one; a vertex when each of its
+// triangles may have its smallest point on an edge that ends there.  A triangle
+// whose f(u) is above the time holds nothing, nor does a rim edge or vertex on a
+// side of the fan that is too far from X for its times.  Every smallest point of the fan
+// passes all of these tests, equal ones too, so what is dropped can neither
+// lower the time nor have been the winner on a tie.
+//
+// Errors: the filter is used where |corr| of every pair of axes is small
+// enough that P's determinant and r keep a quarter of their leading product
+// (A's entries are off by 1e-6 relative, P^-1 by 1e-5, s by 2e-4 s), where r is
+// at least 1e-3 of A.xx and A.yy, and where the triangle's source times are
+// within 1e4 of sqrt(A.xx), sqrt(A.yy) of each other (their differences are off
+// by 1e-3 of those); it takes s off by up to 1e-3 (1 + s) and u by 0.01 plus
+// 1e-4 n |h|, in units of the spacings.  Elsewhere every candidate is kept.
+// What is kept runs through the FP64 candidates in the order of their ids, each
+// lane its own list, so the time and the winner are the same bits.
+//
+// float32 fields do not take this path: their times are rounded to 1e-7 of
+// their own size, so candidates that the filter tells apart often tie.
+// ---------------------------------------------------------------------------
+__host__ __device__ __forceinline__ float ell_rsqrt(float x)
+{
+#ifdef __CUDA_ARCH__
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+#else
+    return 1.0f / sqrtf(x);
+#endif
+}
+__host__ __device__ __forceinline__ float ell_rcp(float x)
+{
+#ifdef __CUDA_ARCH__
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+#else
+    return 1.0f / x;
+#endif
+}
+__host__ __device__ __forceinline__ bool ell_any(bool p)
+{
+#ifdef __CUDA_ARCH__
+    return __any_sync(0xffffffffu, p);
+#else
+    return p;
+#endif
+}
+__host__ __device__ __forceinline__ int ell_low(unsigned m)
+{
+#ifdef __CUDA_ARCH__
+    return __ffs((int)m) - 1;
+#else
+    return __builtin_ctz(m);
+#endif
+}
+
+// m[k] for a k that is the same in the whole launch (selects, not memory).
+__host__ __device__ __forceinline__ double ell_pick(const double m[6], int k)
+{
+    const double a = k == 0 ? m[0] : m[1], b = k == 2 ? m[2] : m[3], c = k == 4 ? m[4] : m[5];
+    return k < 2 ? a : k < 4 ? b : c;
+}
+
+// ell_local in float to a few ulp, from the medium's values v (the six metric
+// words in local order, or s, eps, nx, ny).
+__host__ __device__ __forceinline__ EllipAT<float> ell_local_f(int kind, const EllipDir &D, const double v[6])
+{
+    const float hx = (float)D.hx, hy = (float)D.hy, hz = (float)D.hz;
+    EllipAT<float> A;
+    if (kind == kParamF64) {
+        const float s = (float)v[0], e = (float)v[1], n0 = (float)v[2], n1 = (float)v[3];
+        const float s2 = s * s, a = s2 * ell_rcp(1.0f + 2.0f * e), b = s2 - a;
+        const float n2 = sqrtf(fmaxf((float)((1.0 - v[2] * v[2]) - v[3] * v[3]), 0.0f));
+        const float x = hx * (D.ixx == 0 ? n0 : D.ixx == 3 ? n1 : n2), y = hy * (D.iyy == 0 ? n0 : D.iyy == 3 ? n1 : n2),
+                    z = hz * (D.izz == 0 ? n0 : D.izz == 3 ? n1 : n2);
+        A.xx = fmaf(b * x, x, a * hx * hx);
+        A.yy = fmaf(b * y, y, a * hy * hy);
+        A.zz = fmaf(b * z, z, a * hz * hz);
+        A.xy = (float)D.sxy * b * x * y;
+        A.xz = (float)D.sxz * b * x * z;
+        A.yz = (float)D.syz * b * y * z;
+    } else {
+        A.xx = (float)v[0] * hx * hx;
+        A.yy = (float)v[1] * hy * hy;
+        A.zz = (float)v[2] * hz * hz;
+        A.xy = (float)D.sxy * (float)v[3] * hx * hy;
+        A.xz = (float)D.sxz * (float)v[4] * hx * hz;
+        A.yz = (float)D.syz * (float)v[5] * hy * hz;
+    }
+    return A;
+}
+
+// The medium's values at cell t, as ell_local_f and ell_local_v take them.
+__host__ __device__ __forceinline__ void ell_values(const EllipMedium &M, const EllipDir &D, long long t, double v[6])
+{
+    if (M.kind == kParamF64) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = ell_ld(static_cast<const double *>(M.m[k]) + t);
+        v[4] = v[5] = 0.0;
+    } else {
+        const float *const *f = reinterpret_cast<const float *const *>(M.m);
+        v[0] = ell_ld(f[D.ixx] + t);
+        v[1] = ell_ld(f[D.iyy] + t);
+        v[2] = ell_ld(f[D.izz] + t);
+        v[3] = ell_ld(f[D.ixy] + t);
+        v[4] = ell_ld(f[D.ixz] + t);
+        v[5] = ell_ld(f[D.iyz] + t);
+    }
+}
+
+// ell_local<double> from the medium's values: the same operations.
+__host__ __device__ __forceinline__ EllipA ell_local_v(int kind, const EllipDir &D, const double v[6])
+{
+    double l[6] = {v[0], v[1], v[2], v[3], v[4], v[5]};  // xx yy zz xy xz yz
+    if (kind == kParamF64) {
+        double m[6];
+        ell_metric_from_param(v[0], v[1], v[2], v[3], m);
+        l[0] = ell_pick(m, D.ixx);
+        l[1] = ell_pick(m, D.iyy);
+        l[2] = ell_pick(m, D.izz);
+        l[3] = ell_pick(m, D.ixy);
+        l[4] = ell_pick(m, D.ixz);
+        l[5] = ell_pick(m, D.iyz);
+    }
+    EllipA A;
+    A.xx = l[0] * D.hx * D.hx;
+    A.yy = l[1] * D.hy * D.hy;
+    A.zz = l[2] * D.hz * D.hz;
+    A.xy = (double)D.sxy * l[3] * D.hx * D.hy;
+    A.xz = (double)D.sxz * l[4] * D.hx * D.hz;
+    A.yz = (double)D.syz * l[5] * D.hy * D.hz;
+    return A;
+}
+
+// Candidates kept by the filter: bit r of each, the rim's r-th vertex, spoke,
+// rim edge and triangle; bit 8 of vert, st.
+struct EllKeep {
+    unsigned vert, spoke, rim, tri;
+    float Eb;  // above the new time's distance from st, +inf if unknown
+};
+
+// c: float(st - s_r) of the rim, E: float(tn - st).
+__host__ __device__ __forceinline__ EllKeep ell_filter(bool active, const float c[8], float E, const EllipAT<float> &A)
+{
+    EllKeep K = {0u, 0u, 0u, 0u, HUGE_VALF};
+    const float cof = A.xx * A.yy - A.xy * A.xy, icof = ell_rcp(cof);
+    const float px = (A.yy * A.xz - A.xy * A.yz) * icof, py = (A.xx * A.yz - A.xy * A.xz) * icof;
+    const float r = A.zz - (A.xz * px + A.yz * py);
+    const float big = fmaxf(A.xx, A.yy), small = fminf(A.xx, A.yy);
+    // every comparison is false for a NaN
+    const bool sane = small > 1e-30f && big < 1e30f && A.zz < 1e30f && cof > 0.25f * (A.xx * A.yy) &&
+                      r > 0.25f * A.zz && r > 1e-3f * big && E > -1e30f;
+    float mx = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) mx = fmaxf(mx, c[k]);
+    float Eb = fmaf(fabsf(E), 1e-6f, E);  // above the new time's distance from st
+    const float sr = r * ell_rsqrt(fmaxf(r, 1e-36f));
+    const float far2 = 1e8f * small;
+    const bool near = active && (!sane || Eb + mx > 0.99f * sr);
+    if (!ell_any(near)) return K;
+    unsigned VA = 0, VB = 0, VC = 0, TR = 0;
+    const bool go = near && sane;
+    // ||X - p|| is at least this on the fan's sides x = 1, y = 1, x = -1, y = -1
+    const float kx = cof * ell_rcp(A.yy), ky = cof * ell_rcp(A.xx);
+    float side[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const float off = (q < 2 ? 1.0f : -1.0f) - ((q & 1) ? py : px), d2 = fmaf(off * off, (q & 1) ? ky : kx, r);
+        side[q] = 0.995f * (d2 * ell_rsqrt(fmaxf(d2, 1e-36f)));
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int ka = (k & 1) ? (k + 1) & 7 : k, kc = (k & 1) ? k : k + 1;  // axis neighbour and corner
+        const float ca = c[ka], cc = c[kc];
+        const bool in = go && Eb + fmaxf(fmaxf(ca, cc), 0.0f) > 0.99f * sr;
+        if (ell_any(in)) {
+            const bool along_x = (ka & 3) == 0;
+            const float sa = (ka < 4) ? 1.0f : -1.0f;                       // sign of the axis neighbour
+            const float sc = (float)(along_x ? ell_rj(kc) : ell_ri(kc));    // and of the corner, across
+            const float ga = -sa * ca, gc = sc * (ca - cc);
+            const float gx = along_x ? ga : gc, gy = along_x ? gc : ga;
+            const float hx = fmaf(A.yy, gx, -(A.xy * gy)) * icof, hy = fmaf(A.xx, gy, -(A.xy * gx)) * icof;
+            const float s = fmaf(gx, hx, gy * hy), ds = fmaf(1e-3f, s, 1e-3f), e = 1.0f - s;
+            const float elo = e - ds, ehi = e + ds;
+            const float bx = gx * px, by = gy * py, base = bx + by;
+            const float tol = 1e-3f * (sr + fabsf(bx) + fabsf(by));
+            const float qlo = fmaxf(elo, 1e-6f), qhi = fmaxf(ehi, 1e-6f);
+            const float rlo = ell_rsqrt(qlo), rhi = ell_rsqrt(qhi);
+            const float n_hi = sr * rlo, n_lo = sr * rhi;
+            const float ux0 = fmaf(-n_lo, hx, px), uy0 = fmaf(-n_lo, hy, py);
+            const float ux1 = fmaf(-n_hi, hx, px), uy1 = fmaf(-n_hi, hy, py);
+            const float m0 = sa * (along_x ? ux0 : uy0), w0 = sc * (along_x ? uy0 : ux0);
+            const float m1 = sa * (along_x ? ux1 : uy1), w1 = sc * (along_x ? uy1 : ux1);
+            // weights of the corner, of the axis neighbour and of st at u, over the range of n
+            const float lc = fminf(w0, w1), la = fminf(m0 - w0, m1 - w1), l0 = 1.0f - fmaxf(m0, m1);
+            const float hc = fmaxf(w0, w1), ha = fmaxf(m0 - w0, m1 - w1), h0 = 1.0f - fminf(m0, m1);
+            const float mg = fmaf(1e-4f * n_hi, fabsf(hx) + fabsf(hy), 0.01f);
+            const bool odd = !(fmaxf(ca * ca, cc * cc) < far2);  // differences too coarse, or not finite
+            const bool late = !odd && elo > 0.0f && base + sr * (qlo * rlo) - tol > Eb;
+            if (in && !late) {
+                const bool vc_ = odd || lc < mg, va_ = odd || la < mg, v0_ = odd || l0 < mg;
+                // u's weight of a vertex may be negative: the opposite edge may hold the smallest point
+                VA |= (unsigned)((k & 1) ? va_ : vc_) << k;
+                VB |= (unsigned)((k & 1) ? vc_ : va_) << k;
+                VC |= (unsigned)(v0_ && (odd || Eb + fmaxf(ca, cc) > side[ka >> 1])) << k;
+                TR |= (unsigned)(odd || (ehi > 0.0f && hc > -mg && ha > -mg && h0 > -mg)) << k;
+                if (!(va_ | vc_ | v0_) && elo > 0.0f) Eb = fminf(Eb, base + sr * (qhi * rhi) + tol);
+            }
+        }
+    }
+    auto prev = [](unsigned m) { return ((m << 1) | (m >> 7)) & 0xffu; };  // of the triangle before
+    K.tri = TR;
+    K.rim = VC;
+    K.spoke = VA & prev(VB);
+    unsigned early = 0;  // rim vertices that are not too far for their times
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const float d = (k & 1) ? fmaxf(side[k >> 1], side[((k + 1) >> 1) & 3]) : side[k >> 1];
+        early |= (unsigned)!(Eb + c[k] < d) << k;
+    }
+    K.vert = ((VA | VC) & prev(VB | VC) & early) | (((VA | VB) == 0xffu) ? 0x100u : 0u);
+    K.Eb = Eb;
+    if (near && !sane) K = {0x1ffu, 0xffu, 0xffu, 0xffu, HUGE_VALF};
+    return K;
+}
+
+// Whether an edge kept by ell_filter still may: its own stationary point in
+// float.  cp, cq: c of its ends (0 for st).  Judged only where the ends' times
+// are within 30 sqrt(a) of st's (a the edge's length squared), which leaves
+// their difference within 4e-6 sqrt(a), and away from den = 0.
+__host__ __device__ __forceinline__ bool ell_edge_may(const EllipAT<float> &A, float Eb, float cp, float cq, int pi,
+                                                      int pj, int qi, int qj)
+{
+    const float x = (float)pi, y = (float)pj, ex = (float)(qi - pi), ey = (float)(qj - pj);
+    const float gx = fmaf(A.xx, ex, A.xy * ey), gy = fmaf(A.xy, ex, A.yy * ey);  // P e
+    const float a = fmaf(ex, gx, ey * gy);
+    const float b = fmaf(ex, A.xz, ey * A.yz) - fmaf(x, gx, y * gy);
+    const float c = A.zz + x * fmaf(A.xx, x, 2.0f * (A.xy * y - A.xz)) + y * fmaf(A.yy, y, -2.0f * A.yz);
+    const float d = cp - cq, dd = d * d, den = a - dd, w = 0.01f * (a + dd);
+    if (!(fmaxf(cp * cp, cq * cq) < 1e3f * a) || fabsf(den) < w) return true;
+    if (den < 0.0f) return false;
+    const float q = fmaxf(fmaf(a, c, -(b * b)), 0.0f) * ell_rcp(den), n = q * ell_rsqrt(fmaxf(q, 1e-36f));
+    const float ia = ell_rcp(a), lam = fmaf(-d, n, b) * ia, mg = fmaf(1e-3f * fabsf(d * n), ia, 0.01f);
+    if (lam < -mg || lam > 1.0f + mg) return false;
+    return !(fmaf(lam, d, n) - cp > Eb + 2e-3f * (n + fabsf(d)));
+}
+
+// And a rim vertex (i, j); cv: its c.
+__host__ __device__ __forceinline__ bool ell_vertex_may(const EllipAT<float> &A, float Eb, float cv, int i, int j)
+{
+    const float x = (float)i, y = (float)j;
+    const float c = A.zz + x * fmaf(A.xx, x, 2.0f * (A.xy * y - A.xz)) + y * fmaf(A.yy, y, -2.0f * A.yz);
+    const float n = c * ell_rsqrt(fmaxf(c, 1e-36f));
+    return !(0.999f * n > Eb + cv);
+}
+
+// x / c from r = RN(1/c) where that is exact (Markstein's two remainder
+// corrections, as div_by_const in fold3d_fast.cuh), else x / c.
+__host__ __device__ __forceinline__ unsigned ell_exp(double x)
+{
+#ifdef __CUDA_ARCH__
+    return ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
+#else
+    unsigned long long b;
+    __builtin_memcpy(&b, &x, sizeof b);
+    return (unsigned)(b >> 52) & 0x7ffu;
+#endif
+}
+__host__ __device__ __forceinline__ double ell_div(double x, double c, double r, bool ok)
+{
+    if (!ok || ell_exp(x) - (1023u - 400u) > 800u) return x / c;
+    double q = x * r;
+    double e = fma(-q, c, x);
+    q = fma(e, r, q);
+    e = fma(-q, c, x);
+    return fma(e, r, q);
+}
+
+// ell_tri and ell_edge for a run-time r without their skips.  The terms that
+// ell_bf multiplies by zero are left out (A is finite here, so they add
+// nothing), and the divisions by one denominator share its reciprocal.
+__host__ __device__ __forceinline__ void ell_try_tri(double &tn, int &win, int r, const EllipA &A, double t0, double ta,
+                                                     double tb)
+{
+    const int q = (r + 1) & 7;
+    const double ai = ell_ri(r), aj = ell_rj(r), bi = ell_ri(q), bj = ell_rj(q);
+    const bool odd = r & 1;                    // a is the corner, b the axis neighbour
+    const bool x = ((odd ? q : r) & 3) == 0;   // that neighbour lies along x
+    const double ci = odd ? ai : bi, cj = odd ? aj : bj;
+    const double pax = x ? A.xx : A.yy;                                   // axis . axis
+    const double pc = (A.xx + A.yy) + 2.0 * (ci * cj) * A.xy;             // corner . corner
+    const double p12 = pax + (ci * cj) * A.xy;                            // axis . corner
+    const double p11 = odd ? pc : pax, p22 = odd ? pax : pc;
+    const double qax = x ? ci * A.xz : cj * A.yz, qc = ci * A.xz + cj * A.yz;
+    const double q1 = odd ? qc : qax, q2 = odd ? qax : qc;
+    const double d1 = ta - t0, d2 = tb - t0;
+    const double det = p11 * p22 - p12 * p12;
+    if (!(det > 0.0)) return;
+    const double u1 = p22 * d1 - p12 * d2, u2 = p11 * d2 - p12 * d1;
+    const double w1 = p22 * q1 - p12 * q2, w2 = p11 * q2 - p12 * q1;
+    const double rd = 1.0 / det;
+    const bool ok = ell_exp(det) - (1023u - 400u) <= 800u && ell_exp(rd) - (1023u - 400u) <= 800u;
+    const double s = ell_div(d1 * u1 + d2 * u2, det, rd, ok);
+    const double rr = A.zz - ell_div(q1 * w1 + q2 * w2, det, rd, ok);
+    if (!(s < 1.0 && rr > 0.0)) return;
+    const double n = sqrt(rr / (1.0 - s));
+    const double l1 = ell_div(w1 - n * u1, det, rd, ok), l2 = ell_div(w2 - n * u2, det, rd, ok);
+    if (l1 > 0.0 && l2 > 0.0 && l1 + l2 < 1.0) {
+        const double cand = t0 + (l1 * d1 + l2 * d2) + n;
+        if (cand < tn) {
+            tn = cand;
+            win = 25 + r;
+        }
+    }
+}
+__host__ __device__ __forceinline__ void ell_try_edge(double &tn, int &win, int id, const EllipA &A, double tp,
+                                                      double tq, int pi, int pj, int qi, int qj)
+{
+    const int ei = qi - pi, ej = qj - pj;
+    const double a = ell_bf(A, ei, ej, 0, ei, ej, 0);
+    const double b = ell_bf(A, ei, ej, 0, -pi, -pj, 1);
+    const double c = ell_bf(A, -pi, -pj, 1, -pi, -pj, 1);
+    const double d = tq - tp;
+    const double den = a - d * d;
+    const double disc = a * c - b * b;
+    if (den > 0.0 && disc > 0.0) {
+        const double n = sqrt(disc / den);
+        const double lam = (b - d * n) / a;
+        if (lam > 0.0 && lam < 1.0) {
+            const double cand = tp + lam * d + n;
+            if (cand < tn) {
+                tn = cand;
+                win = id;
+            }
+        }
+    }
+}
+
+// New signed value of the target at field index t whose stored value is `told`
+// from the nine previous-plane magnitudes (rim order, st last), and the winning
+// candidate (-1: none).  Every lane of the warp calls it; a lane that is not
+// `active` changes nothing.  sh: scratch of nine doubles, `stride` elements
+// apart (shared memory on the device).
+__host__ __device__ __forceinline__ double ell_update_fan(bool active, double told, const double (&s)[9],
+                                                          const double (&v)[6], int kind, const EllipDir &D, double *sh,
+                                                          int stride, int &win)
+{
+    const double st = s[8];
+    double tn = fabs(told);
+    win = -1;
+    float c[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        c[r] = (float)(st - s[r]);
+        sh[r * stride] = s[r];
+    }
+    sh[8 * stride] = st;
+    const EllipAT<float> Af = ell_local_f(kind, D, v);
+    const EllKeep K = ell_filter(active, c, (float)(tn - st), Af);
+    if (ell_any((K.vert | K.spoke | K.rim | K.tri) != 0)) {
+        const bool known = K.Eb < HUGE_VALF;
+        unsigned vert = K.vert & 0xffu, edge = 0;
+        for (unsigned m = vert; ell_any(m != 0);) {
+            if (m) {
+                const int r = ell_low(m);
+                m &= m - 1;
+                if (known && !ell_vertex_may(Af, K.Eb, (float)(st - sh[r * stride]), ell_ri(r), ell_rj(r))) vert &= ~(1u << r);
+            }
+        }
+        for (unsigned m = K.spoke | (K.rim << 8); ell_any(m != 0);) {
+            if (m) {
+                const int k = ell_low(m), r = k & 7, q = (k < 8) ? r : (r + 1) & 7;
+                m &= m - 1;
+                const bool spoke = k < 8;
+                if (!known || ell_edge_may(Af, K.Eb, spoke ? 0.0f : (float)(st - sh[r * stride]), (float)(st - sh[q * stride]),
+                                           spoke ? 0 : ell_ri(r), spoke ? 0 : ell_rj(r), ell_ri(q), ell_rj(q)))
+                    edge |= 1u << k;
+            }
+        }
+        if (ell_any((vert | edge | K.tri | (K.vert >> 8)) != 0)) {
+            const EllipA A = ell_local_v(kind, D, v);
+            const bool finite = fabs(A.xx) + fabs(A.yy) + fabs(A.zz) + fabs(A.xy) + fabs(A.xz) + fabs(A.yz) < 1e300;
+            if (K.vert >> 8) ell_vertex(tn, win, 0, A, 0.0, st, 0, 0);
+            while (ell_any(vert != 0)) {
+                if (vert) {
+                    const int r = ell_low(vert);
+                    vert &= vert - 1;
+                    ell_vertex(tn, win, 1 + r, A, 0.0, sh[r * stride], ell_ri(r), ell_rj(r));
+                }
+            }
+            while (ell_any(edge != 0)) {
+                if (edge) {
+                    const int k = ell_low(edge), r = k & 7, q = (k < 8) ? r : (r + 1) & 7;
+                    edge &= edge - 1;
+                    const bool spoke = k < 8;
+                    ell_try_edge(tn, win, 9 + k, A, spoke ? st : sh[r * stride], sh[q * stride], spoke ? 0 : ell_ri(r),
+                                 spoke ? 0 : ell_rj(r), ell_ri(q), ell_rj(q));
+                }
+            }
+            unsigned tri = K.tri;
+            while (ell_any(tri != 0)) {
+                if (tri) {
+                    const int r = ell_low(tri), q = (r + 1) & 7;
+                    tri &= tri - 1;
+                    if (finite) ell_try_tri(tn, win, r, A, st, sh[r * stride], sh[q * stride]);
+                    else ell_tri(tn, win, 25 + r, A, 0.0, st, sh[r * stride], sh[q * stride], ell_ri(r), ell_rj(r),
+                                 ell_ri(q), ell_rj(q));
+                }
+            }
+        }
+    }
+    return ((told > 0.0) ? 1.0 : -1.0) * tn;
+}
 #endif  // __CUDACC__
 
 }  // namespace fold3d

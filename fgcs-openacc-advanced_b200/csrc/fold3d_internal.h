@@ -98,9 +98,12 @@ enum Variant {
 #endif
 constexpr unsigned kPollNs = FOLD3D_POLL_NS;
 
-// Items a batched pass's CTA claims at a time (1..32); build option.
+// Items a batched pass's CTA claims at a time (1..32); build option.  24
+// instances of 96 to 200 points per axis to 1e-10, for 1, 2, 4 and 8: 297, 274,
+// 327, 498 ms: fewer, and every item pays for the claim and the instance; more,
+// and items that others wait for stand in a queue.
 #ifndef FOLD3D_BATCH_CHUNK
-#define FOLD3D_BATCH_CHUNK 4
+#define FOLD3D_BATCH_CHUNK 2
 #endif
 constexpr int kBatchChunk = FOLD3D_BATCH_CHUNK;
 static_assert(kBatchChunk >= 1 && kBatchChunk <= 32, "batch chunk");
@@ -124,28 +127,27 @@ constexpr int kWaveTV = FOLD3D_WAVE_TV;
 // count that measured fastest.  Drift: 4 (128 registers; ms at 512^3, 8 sweeps,
 // and 1280^3, 2 sweeps, for 3, 4, 5 and 6: 342, 342, 333, 352 and 1269, 1126,
 // 1158, 1168): the update is one long chain per point, which spills and
-// reloads below 100 registers lengthen.  The FP64 elliptical medium 6, and 7 on
-// large planes; the float32 one 8; batched solves (many small instances) 8.
+// reloads below 100 registers lengthen.  The FP64 elliptical medium 5 (128^3
+// and 512^3 to 1e-10, for 4, 5 and 6: 12.7, 12.7, 13.0 and 317, 312, 328); the
+// float32 one 8; FP64 batches 5 (24 instances of 96 to 200 points per axis, for
+// 4, 5, 6 and 8: 327, 327, 340, 377), float32 batches 8.
 #ifndef FOLD3D_WAVE_MINB_DRIFT
 #define FOLD3D_WAVE_MINB_DRIFT 4
 #endif
 #ifndef FOLD3D_WAVE_MINB_ELLIP
-#define FOLD3D_WAVE_MINB_ELLIP 6
+#define FOLD3D_WAVE_MINB_ELLIP 5
 #endif
 #ifndef FOLD3D_WAVE_MINB_ELLIP_F32
 #define FOLD3D_WAVE_MINB_ELLIP_F32 8
 #endif
 #ifndef FOLD3D_WAVE_MINB_BATCH
-#define FOLD3D_WAVE_MINB_BATCH 8
+#define FOLD3D_WAVE_MINB_BATCH 5
 #endif
-#ifndef FOLD3D_WAVE_MINB_LARGE
-#define FOLD3D_WAVE_MINB_LARGE 8  // large planes, float32 elliptical medium
-#endif
-#ifndef FOLD3D_WAVE_MINB_LARGE_ELLIP
-#define FOLD3D_WAVE_MINB_LARGE_ELLIP 7
+#ifndef FOLD3D_WAVE_MINB_BATCH_F32
+#define FOLD3D_WAVE_MINB_BATCH_F32 8
 #endif
 #ifndef FOLD3D_WAVE_LARGE_TILES
-#define FOLD3D_WAVE_LARGE_TILES 8192
+#define FOLD3D_WAVE_LARGE_TILES 1536
 #endif
 constexpr int kLargePlaneTiles = FOLD3D_WAVE_LARGE_TILES;
 static_assert(kWaveTV == 1 || kWaveTV == 2 || kWaveTV == 4 || kWaveTV == 8, "tile rows");
@@ -206,14 +208,14 @@ constexpr unsigned kNoWinner = 0xffu;
 struct EllipDir;     // fold3d_ellip.cuh
 struct EllipParam;   // below, once EllipDir is complete
 
-// A pass of the drift medium over tiles of tv rows (1, 2, 4 or 8).
+// A pass of the drift medium over tiles of tv rows (1, 2 or 4).
 cudaError_t launch_wave_pass(double *T, const WaveArgs &a, const DirTable &tab, int tv, int grid, cudaStream_t s);
-int drift_blocks_per_sm(int tv);
 // The elliptical medium's field is double, or float when f32.  large: the
 // variant compiled for passes over large planes (kLargePlaneTiles).
 cudaError_t launch_wave_pass_ellip(void *T, bool f32, const WaveArgs &a, const EllipParam &p, int grid, cudaStream_t s,
-                                   bool large = false);
+                                   bool large);
 int wave_blocks_per_sm(bool f32, bool large);
+int drift_blocks_per_sm(int tv);
 
 }  // namespace fold3d
 #include "fold3d_ellip.cuh"

@@ -60,37 +60,44 @@ __device__ __forceinline__ bool bits_differ(float a, float b) { return __float_a
 constexpr int kWaveThreads = 128;  // four warps
 
 
-template <int MED, class R, bool LARGE> constexpr int wave_min_blocks()
+template <class R> constexpr int wave_min_blocks()
 {
-    return LARGE ? (sizeof(R) == 8 ? FOLD3D_WAVE_MINB_LARGE_ELLIP : FOLD3D_WAVE_MINB_LARGE)
-                 : (sizeof(R) == 8 ? FOLD3D_WAVE_MINB_ELLIP : FOLD3D_WAVE_MINB_ELLIP_F32);
+    return sizeof(R) == 8 ? FOLD3D_WAVE_MINB_ELLIP : FOLD3D_WAVE_MINB_ELLIP_F32;
 }
 
-// Medium-dependent launch parameters: the drift medium's constant table, or
-// the elliptical medium's direction constants and metric arrays.
-template <int MED> struct WaveMedium;
-template <> struct WaveMedium<kMediumDrift> {
-    using type = DirTable;
-};
-template <> struct WaveMedium<kMediumEllip> {
-    using type = EllipParam;
-};
-
 // A lane's point (u, v) of the target plane src + sg: update it from the source
-// plane and store it; whether it changed.
+// plane and store it; whether it changed.  All lanes of the warp call this
+// together; points outside the plane are left out.  sh: the thread's scratch
+// (ell_update_fan), `stride` doubles apart; unused by float fields.
 template <class R>
 __device__ __forceinline__ bool ellip_point(R *__restrict__ T, const WaveArgs &a, const EllipParam &tab, int src, int u,
-                                            int v, double &dmax, unsigned &evaluated)
+                                            int v, double *sh, int stride, double &dmax, unsigned &evaluated)
 {
     const PlaneGeom &g = a.pg;
-    if (u > g.nu || v > g.nv) return false;
+    const bool active = u <= g.nu && v <= g.nv;
     const long long s = (long long)src * g.s_nrm + (long long)u * g.su + (long long)v * g.sv, d = s + g.sn;
-    const R told = ld_cg(T + d), st = fabs(ld_cg(T + s));
-    R nb[8];
+    R told = R(0), tnew = R(0), fan[9] = {};
+    int win = -1;
+    if constexpr (sizeof(R) == 8) {
+        double m[6] = {};
+        if (active) {
+            ell_values(tab.med, tab.dir, d, m);
+            told = ld_cg(T + d);
+            fan[8] = fabs(ld_cg(T + s));
 #pragma unroll
-    for (int r = 0; r < 8; ++r) nb[r] = fabs(ld_cg(T + s + ell_ri(r) * g.sx + ell_rj(r) * g.sy));
-    int win;
-    const R tnew = point_update_ellip(told, st, nb, ell_local<R>(tab.med, tab.dir, d), win);
+            for (int r = 0; r < 8; ++r) fan[r] = fabs(ld_cg(T + s + ell_ri(r) * g.sx + ell_rj(r) * g.sy));
+        }
+        tnew = ell_update_fan(active, told, fan, m, tab.med.kind, tab.dir, sh, stride, win);
+        if (!active) return false;
+    } else {
+        if (!active) return false;
+        told = ld_cg(T + d);
+        fan[8] = fabs(ld_cg(T + s));
+        R nb[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) nb[r] = fabs(ld_cg(T + s + ell_ri(r) * g.sx + ell_rj(r) * g.sy));
+        tnew = point_update_ellip(told, fan[8], nb, ell_local<R>(tab.med, tab.dir, d), win);
+    }
     ++evaluated;
     if (!bits_differ(tnew, told)) return false;
     if (a.winners) a.winners[d] = (win < 0) ? (unsigned char)kNoWinner : (unsigned char)(a.dir * kEllipCands + win);
@@ -133,10 +140,10 @@ __device__ __forceinline__ int wave_div(int x, int n, float inv, int &r)
 // publish its flag.  Adds each changed point's |dT| into dmax and the
 // evaluated points into evaluated.  Returns false if a wait gave up (the
 // item is then left unpublished and the caller must leave).
-template <int MED, class R, int TV = kWaveTV>
+template <class R, int TV>
 __device__ __forceinline__ bool wave_item(R *__restrict__ T, const WaveArgs &a,
-                                          const typename WaveMedium<MED>::type &tab, int item, double &dmax,
-                                          unsigned &evaluated)
+                                          const EllipParam &tab, int item, double *sh,
+                                          double &dmax, unsigned &evaluated)
 {
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
@@ -172,7 +179,7 @@ __device__ __forceinline__ bool wave_item(R *__restrict__ T, const WaveArgs &a,
     if (!skip) {
         const int u = tu * 32 + lane + 1;
         const int v = tv * TV + warp + 1;
-        if (ellip_point<R>(T, a, tab, src, u, v, dmax, evaluated)) {
+        if (ellip_point<R>(T, a, tab, src, u, v, sh, 32 * TV, dmax, evaluated)) {
             changed = 1;
             wave_mark<1, TV>(a, u, v, tgt);
             wave_mark<2, TV>(a, u, v, tgt);
@@ -211,6 +218,91 @@ __device__ __forceinline__ void wave_flush(double d, unsigned long long e, unsig
     __syncthreads();
 }
 
+// The items of a pass whose warps work alone: every warp claims and publishes
+// whole items of 32 x TV points, each with one fence; no warp waits at a CTA
+// barrier for another's rows.  rows(src, u, v0, last, active, prefetch) updates
+// the lane's points (u, v0 .. v0 + last - 1) of a tile (lanes that are not
+// active only keep company), calls prefetch() once its first loads are under
+// way, and returns the changed ones of the lane's points as bits.  The change
+// marks of the other orientations (32 scattered stores) come after the item is
+// published, for the fence would wait for them.
+template <int TV, class Rows> __device__ __forceinline__ void warp_items(const WaveArgs &a, Rows rows)
+{
+    const int lane = threadIdx.x & 31;
+    const int ntiles = a.ntu * a.ntv;
+    const unsigned total = (unsigned)(a.steps * ntiles);
+    const float inv_tiles = 1.0f / (float)ntiles, inv_ntu = 1.0f / (float)a.ntu;
+    const unsigned want = a.epoch << 1;  // flags hold (pass << 1) | changed
+    const bool may_skip = a.epoch >= a.skip_from;
+    // Lanes 0..8 each watch one tile of an item's 3 x 3 neighbourhood: its
+    // change mark from earlier passes, and its step p-1 flag (which also says
+    // whether that item changed the source plane).  watch() gives the lane's
+    // flag, or NULL where there is nothing to wait for.
+    auto watch = [&](unsigned item, int &p, int &t, int &tu, int &tv, bool &recent) -> const unsigned * {
+        p = wave_div((int)item, ntiles, inv_tiles, t);
+        tv = wave_div(t, a.ntu, inv_ntu, tu);
+        const int nu = tu + lane % 3 - 1, nv = tv + lane / 3 - 1, nt = nv * a.ntu + nu;
+        const bool in = lane < 9 && nu >= 0 && nu < a.ntu && nv >= 0 && nv < a.ntv;
+        recent = in && may_skip && __ldcg(a.mod[0] + (long long)(a.first_src + p * a.sg) * ntiles + nt) + 5u >= a.epoch;
+        return (in && p > 0) ? a.flags + (long long)(p - 1) * ntiles + nt : nullptr;
+    };
+    // The warp holds two claimed items: the flags of the second are read while
+    // the first is worked on, and the fence that publishes the first also
+    // orders that read before the second's loads.  A skipped item has written
+    // nothing, so its flag needs no fence (who waits for it reads what earlier
+    // passes left); the next item that is not skipped then fences first.
+    unsigned ahead = 0;
+    if (lane == 0) ahead = atomicAdd(a.work, 1u);
+    unsigned item = __shfl_sync(0xffffffffu, ahead, 0);
+    if (lane == 0) ahead = atomicAdd(a.work, 1u);
+    int p = 0, t = 0, tu = 0, tv = 0;
+    bool recent = false;
+    const unsigned *fl = item < total ? watch(item, p, t, tu, tv, recent) : nullptr;
+    unsigned f = 0;
+    bool fenced = true;  // nothing has been read relaxed since the last fence
+    while (item < total) {
+        bool gave_up = false;
+        if (fl && f < want) {
+            f = wait_flag(fl, want, a.status, a.timeout_ns);
+            gave_up = f == 0;
+        }
+        recent |= fl && (f & 1u);
+        if (__any_sync(0xffffffffu, gave_up)) break;
+        const bool skip = may_skip && !__any_sync(0xffffffffu, recent);
+        const unsigned next = __shfl_sync(0xffffffffu, ahead, 0);
+        if (lane == 0) ahead = atomicAdd(a.work, 1u);
+        const int src = a.first_src + p * a.sg, tgt = src + a.sg, u = tu * 32 + lane + 1, v0 = tv * TV + 1;
+        const int t0 = t;
+        auto prefetch = [&] {
+            if (next < total) {
+                fl = watch(next, p, t, tu, tv, recent);
+                f = fl ? ld_relaxed(fl) : 0u;
+            }
+        };
+        unsigned changed = 0, any = 0;
+        if (!skip) {
+            if (!fenced) fence_acq_rel();
+            changed = rows(src, u, v0, min(TV, a.pg.nv - v0 + 1), u <= a.pg.nu, prefetch);
+            any = __any_sync(0xffffffffu, changed != 0) ? 1u : 0u;
+            __syncwarp();
+            fence_acq_rel();
+        } else {
+            prefetch();
+        }
+        fenced = !skip;
+        if (lane == 0) st_relaxed(a.flags + item, want | any);
+        __syncwarp();
+        if (changed) {
+            wave_mark<1, TV>(a, u, v0, tgt);
+#pragma unroll
+            for (int r = 0; r < TV; ++r)
+                if ((changed >> r) & 1u) wave_mark<2, TV>(a, u, v0 + r, tgt);
+        }
+        if (any && lane == 0) a.mod[0][(long long)tgt * ntiles + t0] = a.epoch;
+        item = next;
+    }
+}
+
 // A pass of the drift medium.  Every warp claims and processes whole items
 // of 32 x TV points on its own, the tile's rows one after another, and
 // publishes them with one fence; no warp waits at a CTA barrier for another's
@@ -234,53 +326,11 @@ __global__ void __launch_bounds__(kWaveThreads, FOLD3D_WAVE_MINB_DRIFT)
     __shared__ float s_dif[9 * kWaveThreads];
     copy_table(s_tab, tab, threadIdx.x, kWaveThreads);
     __syncthreads();
-    const PlaneGeom &g = a.pg;
-    const int lane = threadIdx.x & 31;
-    const int ntiles = a.ntu * a.ntv;
-    const unsigned total = (unsigned)(a.steps * ntiles);
-    const float inv_tiles = 1.0f / (float)ntiles, inv_ntu = 1.0f / (float)a.ntu;
-    const unsigned want = a.epoch << 1;  // flags hold (pass << 1) | changed
-    const bool may_skip = a.epoch >= a.skip_from;
     double dmax = 0.0;
     unsigned evaluated = 0;
-    // Lanes 0..8 each watch one tile of an item's 3 x 3 neighbourhood: its
-    // change mark from earlier passes, and its step p-1 flag (which also says
-    // whether that item changed the source plane).  watch() gives the lane's
-    // flag, or NULL where there is nothing to wait for.
-    auto watch = [&](unsigned item, int &p, int &t, int &tu, int &tv, bool &recent) -> const unsigned * {
-        p = wave_div((int)item, ntiles, inv_tiles, t);
-        tv = wave_div(t, a.ntu, inv_ntu, tu);
-        const int nu = tu + lane % 3 - 1, nv = tv + lane / 3 - 1, nt = nv * a.ntu + nu;
-        const bool in = lane < 9 && nu >= 0 && nu < a.ntu && nv >= 0 && nv < a.ntv;
-        recent = in && may_skip && __ldcg(a.mod[0] + (long long)(a.first_src + p * a.sg) * ntiles + nt) + 5u >= a.epoch;
-        return (in && p > 0) ? a.flags + (long long)(p - 1) * ntiles + nt : nullptr;
-    };
-    // The warp holds two claimed items: the flags of the second are read while
-    // the first is worked on, and the fence that publishes the first also
-    // orders that read before the second's loads.
-    unsigned ahead = 0;
-    if (lane == 0) ahead = atomicAdd(a.work, 1u);
-    unsigned item = __shfl_sync(0xffffffffu, ahead, 0);
-    if (lane == 0) ahead = atomicAdd(a.work, 1u);
-    int p = 0, t = 0, tu = 0, tv = 0;
-    bool recent = false;
-    const unsigned *fl = item < total ? watch(item, p, t, tu, tv, recent) : nullptr;
-    unsigned f = 0;
-    while (item < total) {
-        bool gave_up = false;
-        if (fl && f < want) {
-            f = wait_flag(fl, want, a.status, a.timeout_ns);
-            gave_up = f == 0;
-        }
-        recent |= fl && (f & 1u);
-        if (__any_sync(0xffffffffu, gave_up)) break;
-        const bool skip = may_skip && !__any_sync(0xffffffffu, recent);
-        const unsigned next = __shfl_sync(0xffffffffu, ahead, 0);
-        if (lane == 0) ahead = atomicAdd(a.work, 1u);
-        const int src = a.first_src + p * a.sg, tgt = src + a.sg, u = tu * 32 + lane + 1, v0 = tv * TV + 1;
-        const int t0 = t, last = min(TV, g.nv - v0 + 1);
+    warp_items<TV>(a, [&](int src, int u, int v0, int last, bool active, auto prefetch) -> unsigned {
+        const PlaneGeom &g = a.pg;
         const double *s = T + ((long long)src * g.s_nrm + (long long)u * g.su + (long long)v0 * g.sv);
-        const bool active = u <= g.nu && !skip;
         // source rows v0 - 1 .. v0 + 1, and the target
         double w[3][3] = {}, told = 0.0;
         if (active) {
@@ -290,65 +340,61 @@ __global__ void __launch_bounds__(kWaveThreads, FOLD3D_WAVE_MINB_DRIFT)
                 for (int j = 0; j < 3; ++j) w[i][j] = fabs(ld_cg(s + (i - 1) * g.sv + (j - 1) * g.su));
             told = ld_cg(s + g.sn);
         }
-        if (next < total) {
-            fl = watch(next, p, t, tu, tv, recent);
-            f = fl ? ld_relaxed(fl) : 0u;
-        }
+        prefetch();
         unsigned any = 0;
-        if (!skip) {
 #pragma unroll 1
-            for (int r = 0; r < last; ++r, s += g.sv) {
-                double w3[3] = {}, told3 = 0.0;  // the next row's new sources and target
-                if (TV > 1 && active && r + 1 < last) {
+        for (int r = 0; r < last; ++r, s += g.sv) {
+            double w3[3] = {}, told3 = 0.0;  // the next row's new sources and target
+            if (TV > 1 && active && r + 1 < last) {
 #pragma unroll
-                    for (int j = 0; j < 3; ++j) w3[j] = fabs(ld_cg(s + 2 * g.sv + (j - 1) * g.su));
-                    told3 = ld_cg(s + g.sv + g.sn);
-                }
-                const double fan[9] = {w[1][2], w[2][2], w[2][1], w[2][0], w[1][0], w[0][0], w[0][1], w[0][2], w[1][1]};
-                const double tnew =
-                    point_update_fan(active, told, fan, s_tab, &s_fan[threadIdx.x], &s_dif[threadIdx.x], kWaveThreads);
-                const bool changed = active && bits_differ(tnew, told);
-                evaluated += active;
-                if (changed) {
-                    const_cast<double *>(s)[g.sn] = tnew;
-                    dmax = fmax(dmax, fabs(tnew - told));
-                    wave_mark<2, TV>(a, u, v0 + r, tgt);
-                }
-                any |= (unsigned)changed;
-                if (TV > 1) {
-#pragma unroll
-                    for (int j = 0; j < 3; ++j) {
-                        w[0][j] = w[1][j];
-                        w[1][j] = w[2][j];
-                        w[2][j] = w3[j];
-                    }
-                    told = told3;
-                }
+                for (int j = 0; j < 3; ++j) w3[j] = fabs(ld_cg(s + 2 * g.sv + (j - 1) * g.su));
+                told3 = ld_cg(s + g.sv + g.sn);
             }
-            if (any) wave_mark<1, TV>(a, u, v0, tgt);
-            any = __any_sync(0xffffffffu, any);
+            const double fan[9] = {w[1][2], w[2][2], w[2][1], w[2][0], w[1][0], w[0][0], w[0][1], w[0][2], w[1][1]};
+            const double tnew =
+                point_update_fan(active, told, fan, s_tab, &s_fan[threadIdx.x], &s_dif[threadIdx.x], kWaveThreads);
+            const bool changed = active && bits_differ(tnew, told);
+            evaluated += active;
+            if (changed) {
+                const_cast<double *>(s)[g.sn] = tnew;
+                dmax = fmax(dmax, fabs(tnew - told));
+            }
+            any |= (unsigned)changed << r;
+            if (TV > 1) {
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    w[0][j] = w[1][j];
+                    w[1][j] = w[2][j];
+                    w[2][j] = w3[j];
+                }
+                told = told3;
+            }
         }
-        __syncwarp();
-        fence_acq_rel();
-        if (lane == 0) {
-            st_relaxed(a.flags + item, want | any);
-            if (any) a.mod[0][(long long)tgt * ntiles + t0] = a.epoch;
-        }
-        __syncwarp();
-        item = next;
-    }
+        return any;
+    });
     __syncthreads();
     wave_flush<kWaveThreads / 32>(dmax, evaluated, a.maxd, a.evaluated);
 }
 
 // A pass of the elliptical medium: the warps of a CTA share each item's rows.
-// (Its point update is long straight-line code; warps that run it together
-// fetch it together.)
-template <int MED, class R, bool LARGE>
-__global__ void __launch_bounds__(kWaveThreads, (wave_min_blocks<MED, R, LARGE>()))
-    wave_pass_kernel(R *__restrict__ T, WaveArgs a, const __grid_constant__ typename WaveMedium<MED>::type tab)
+// (Its update is 700 instructions of mostly straight code; warps that run it
+// together fetch it together.  With items of their own, as in the drift
+// medium's passes, 512^3 to 1e-10 took 437 ms instead of 312.)
+//
+// wave_pass_kernel is for planes of kLargePlaneTiles tiles or more, where a CTA
+// has several items of a step: two barriers per item.  Before the first, warp 0
+// watches the item's dependencies and the last warp claims the next item; the
+// rows run between them; after the second, warp 1 publishes the item while the
+// others go on.  On smaller planes, and for float fields, the plane-to-plane
+// chain binds and wave_item_kernel is faster, where thread 0 publishes before
+// anything of the next item begins (ms; two barriers, this: 128^3 to 1e-10
+// 12.7, 12.2; 512^3 312, 339; float32 380x319x257 72.4, 69.8).
+template <class R>
+__global__ void __launch_bounds__(kWaveThreads, wave_min_blocks<R>())
+    wave_item_kernel(R *__restrict__ T, WaveArgs a, const __grid_constant__ EllipParam tab)
 {
     __shared__ int s_next;
+    __shared__ double s_fan[sizeof(R) == 8 ? 9 * kWaveThreads : 1];
     const long long total = (long long)a.steps * a.ntu * a.ntv;
     double dmax = 0.0;
     unsigned evaluated = 0;
@@ -365,9 +411,81 @@ __global__ void __launch_bounds__(kWaveThreads, (wave_min_blocks<MED, R, LARGE>(
             const unsigned w = atomicAdd(a.work, 1u);
             s_next = (w < total) ? (int)w : -1;
         }
-        if (!wave_item<MED, R, kWaveTV>(T, a, tab, item, dmax, evaluated)) break;
+        if (!wave_item<R, kWaveTV>(T, a, tab, item, s_fan + threadIdx.x, dmax, evaluated)) break;
     }
     wave_flush<kWaveTV>(dmax, evaluated, a.maxd, a.evaluated);
+}
+
+__global__ void __launch_bounds__(kWaveThreads, wave_min_blocks<double>())
+    wave_pass_kernel(double *__restrict__ T, WaveArgs a, const __grid_constant__ EllipParam tab)
+{
+    constexpr int TV = kWaveTV, kWarps = kWaveThreads / 32;
+    static_assert(kWarps == TV && TV >= 3, "one row per warp");
+    __shared__ int s_item[2];           // the CTA's items, by parity; -1 for none
+    __shared__ int s_state;             // 0 update, 1 skip, 2 a wait gave up
+    __shared__ double s_fan[9 * kWaveThreads];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int ntiles = a.ntu * a.ntv;
+    const unsigned total = (unsigned)(a.steps * ntiles);
+    const float inv_tiles = 1.0f / (float)ntiles, inv_ntu = 1.0f / (float)a.ntu;
+    const unsigned want = a.epoch << 1;  // flags hold (pass << 1) | changed
+    const bool may_skip = a.epoch >= a.skip_from;
+    double dmax = 0.0;
+    unsigned evaluated = 0;
+    if (threadIdx.x == 0) {
+        const unsigned w = atomicAdd(a.work, 1u);
+        s_item[0] = (w < total) ? (int)w : -1;
+    }
+    __syncthreads();
+    for (int q = 0;; ++q) {
+        const int slot = q & 1, item = s_item[slot];
+        if (item < 0) break;
+        int t, tu;
+        const int p = wave_div(item, ntiles, inv_tiles, t), tv = wave_div(t, a.ntu, inv_ntu, tu);
+        const int src = a.first_src + p * a.sg, tgt = src + a.sg, u = tu * 32 + lane + 1;
+        if (warp == 0) {
+            // lanes 0..8 each watch one tile of the 3 x 3 neighbourhood: its
+            // change mark from earlier passes, and its step p-1 flag (which
+            // also says whether that item changed the source plane)
+            const int nu = tu + lane % 3 - 1, nv = tv + lane / 3 - 1;
+            bool gave_up = false, recent = false;
+            if (lane < 9 && nu >= 0 && nu < a.ntu && nv >= 0 && nv < a.ntv) {
+                const int nt = nv * a.ntu + nu;
+                if (may_skip) recent = __ldcg(a.mod[0] + (long long)src * ntiles + nt) + 5u >= a.epoch;
+                if (p > 0) {
+                    const unsigned f =
+                        wait_flag(a.flags + (long long)(p - 1) * ntiles + nt, want, a.status, a.timeout_ns);
+                    gave_up = f == 0;
+                    recent |= f & 1u;
+                }
+            }
+            gave_up = __any_sync(0xffffffffu, gave_up);
+            recent = __any_sync(0xffffffffu, recent);
+            if (lane == 0) s_state = gave_up ? 2 : (may_skip && !recent) ? 1 : 0;
+        }
+        unsigned claim = 0;  // the next item; looked at only after this one's rows
+        const bool claims = threadIdx.x == 32 * (kWarps - 1);
+        if (claims) claim = atomicAdd(a.work, 1u);
+        __syncthreads();
+        const int state = s_state;
+        if (state == 2) break;
+        bool changed = false;
+        if (state == 0)
+            changed = ellip_point<double>(T, a, tab, src, u, tv * TV + warp + 1, s_fan + threadIdx.x, kWaveThreads, dmax,
+                                     evaluated);
+        if (changed) {
+            wave_mark<1, TV>(a, u, tv * TV + warp + 1, tgt);
+            wave_mark<2, TV>(a, u, tv * TV + warp + 1, tgt);
+        }
+        if (claims) s_item[slot ^ 1] = (claim < total) ? (int)claim : -1;
+        const bool any = __syncthreads_or(changed);  // precedes the release: every thread's stores come before the flag
+        if (threadIdx.x == 32) {
+            st_release(a.flags + item, want | (any ? 1u : 0u));
+            if (any) a.mod[0][(long long)tgt * ntiles + t] = a.epoch;
+        }
+    }
+    __syncthreads();
+    wave_flush<kWarps>(dmax, evaluated, a.maxd, a.evaluated);
 }
 
 // ---------------------------------------------------------------------------
@@ -379,12 +497,15 @@ __global__ void __launch_bounds__(kWaveThreads, (wave_min_blocks<MED, R, LARGE>(
 // same instance) come earlier in that order, and the launch's claimed items
 // spread over many instances at once.
 // ---------------------------------------------------------------------------
-// Resident CTAs per SM the batched kernel is compiled for, by tile height:
-// the same register budget per thread (65536 / (128 * 8)) for every height.
-template <int TV> constexpr int batch_min_blocks() { return FOLD3D_WAVE_MINB_BATCH * kWaveTV / TV; }
+// Resident CTAs per SM the batched kernel is compiled for, by tile height: the
+// same register budget per thread for every height.
+template <class R, int TV> constexpr int batch_min_blocks()
+{
+    return (sizeof(R) == 8 ? FOLD3D_WAVE_MINB_BATCH : FOLD3D_WAVE_MINB_BATCH_F32) * 4 / TV;
+}
 
 template <class R, int TV>
-__global__ void __launch_bounds__(32 * TV, batch_min_blocks<TV>()) batch_pass_kernel(BatchArgs b)
+__global__ void __launch_bounds__(32 * TV, batch_min_blocks<R, TV>()) batch_pass_kernel(BatchArgs b)
 {
     // A CTA claims kBatchChunk consecutive items at a time, and the first
     // lanes of warp 0 locate them in parallel (two binary searches each over
@@ -398,6 +519,7 @@ __global__ void __launch_bounds__(32 * TV, batch_min_blocks<TV>()) batch_pass_ke
     __shared__ int s_n;     // items of the current chunk
     __shared__ int s_cur;   // the active slot staged in s_inst, -1 for none
     __shared__ BatchInst s_inst;
+    __shared__ double s_fan[sizeof(R) == 8 ? 9 * 32 * TV : 1];
     const unsigned total = *b.total;
     if (threadIdx.x == 0) {
         const unsigned w = atomicAdd(b.work, (unsigned)kBatchChunk);
@@ -447,8 +569,8 @@ __global__ void __launch_bounds__(32 * TV, batch_min_blocks<TV>()) batch_pass_ke
             }
             __syncthreads();
         }
-        if (!wave_item<kMediumEllip, R, TV>(static_cast<R *>(s_inst.T), s_inst.a, s_inst.p, s_loc[q][1], dmax,
-                                            evaluated))
+        if (!wave_item<R, TV>(static_cast<R *>(s_inst.T), s_inst.a, s_inst.p, s_loc[q][1],
+                                            s_fan + threadIdx.x, dmax, evaluated))
             break;
     }
     if (s_cur >= 0) wave_flush<TV>(dmax, evaluated, s_inst.a.maxd, s_inst.a.evaluated);
@@ -545,7 +667,6 @@ cudaError_t launch_wave_pass(double *T, const WaveArgs &a, const DirTable &tab, 
     case 1: drift_pass_kernel<1><<<grid, kWaveThreads, 0, s>>>(T, a, tab); break;
     case 2: drift_pass_kernel<2><<<grid, kWaveThreads, 0, s>>>(T, a, tab); break;
     case 4: drift_pass_kernel<4><<<grid, kWaveThreads, 0, s>>>(T, a, tab); break;
-    case 8: drift_pass_kernel<8><<<grid, kWaveThreads, 0, s>>>(T, a, tab); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
@@ -554,15 +675,9 @@ cudaError_t launch_wave_pass(double *T, const WaveArgs &a, const DirTable &tab, 
 cudaError_t launch_wave_pass_ellip(void *T, bool f32, const WaveArgs &a, const EllipParam &p, int grid, cudaStream_t s,
                                    bool large)
 {
-    float *tf = static_cast<float *>(T);
-    double *td = static_cast<double *>(T);
-    if (f32) {
-        if (large) wave_pass_kernel<kMediumEllip, float, true><<<grid, kWaveThreads, 0, s>>>(tf, a, p);
-        else wave_pass_kernel<kMediumEllip, float, false><<<grid, kWaveThreads, 0, s>>>(tf, a, p);
-    } else {
-        if (large) wave_pass_kernel<kMediumEllip, double, true><<<grid, kWaveThreads, 0, s>>>(td, a, p);
-        else wave_pass_kernel<kMediumEllip, double, false><<<grid, kWaveThreads, 0, s>>>(td, a, p);
-    }
+    if (f32) wave_item_kernel<float><<<grid, kWaveThreads, 0, s>>>(static_cast<float *>(T), a, p);
+    else if (large) wave_pass_kernel<<<grid, kWaveThreads, 0, s>>>(static_cast<double *>(T), a, p);
+    else wave_item_kernel<double><<<grid, kWaveThreads, 0, s>>>(static_cast<double *>(T), a, p);
     return cudaGetLastError();
 }
 
@@ -575,17 +690,14 @@ template <class K> static int occupancy(K kernel)
 
 int wave_blocks_per_sm(bool f32, bool large)
 {
-    if (f32)
-        return large ? occupancy(wave_pass_kernel<kMediumEllip, float, true>)
-                     : occupancy(wave_pass_kernel<kMediumEllip, float, false>);
-    return large ? occupancy(wave_pass_kernel<kMediumEllip, double, true>)
-                 : occupancy(wave_pass_kernel<kMediumEllip, double, false>);
+    return f32 ? occupancy(wave_item_kernel<float>) : large ? occupancy(wave_pass_kernel)
+                                                            : occupancy(wave_item_kernel<double>);
 }
 
 int drift_blocks_per_sm(int tv)
 {
     return tv == 1 ? occupancy(drift_pass_kernel<1>) : tv == 2 ? occupancy(drift_pass_kernel<2>)
-         : tv == 8 ? occupancy(drift_pass_kernel<8>) : occupancy(drift_pass_kernel<4>);
+                                                               : occupancy(drift_pass_kernel<4>);
 }
 
 }  // namespace fold3d
