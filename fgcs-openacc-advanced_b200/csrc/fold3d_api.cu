@@ -169,6 +169,7 @@ struct fold3d_ctx {
     fold3d_grid key_wg{};
     int key_wtv = 0;                         // and tiles of this many rows
     unsigned *w_flags = nullptr;
+    int w_fshift = 0;                        // log2 of the words between two flags
     unsigned *w_mod[3] = {nullptr, nullptr, nullptr};
     unsigned *w_counters = nullptr;          // [0] work, [1] status
     unsigned long long *w_evaluated = nullptr;
@@ -446,6 +447,8 @@ static int wave_scratch(fold3d_ctx *c, const fold3d_grid &g, int tv)
             (e = cudaMemset(c->w_mod[b], 0, words * 4)) != cudaSuccess)
             return set_errorf(FOLD3D_ERR_NOMEM, "wavefront scratch: %s", cudaGetErrorString(e));
     }
+    c->w_fshift = (long long)flag_words <= kSpreadFlags ? 3 : 0;
+    flag_words <<= c->w_fshift;
     if ((e = cudaMalloc(&c->w_flags, flag_words * 4)) != cudaSuccess ||
         (e = cudaMemset(c->w_flags, 0, flag_words * 4)) != cudaSuccess)
         return set_errorf(FOLD3D_ERR_NOMEM, "wavefront scratch: %s", cudaGetErrorString(e));
@@ -518,6 +521,7 @@ static int solve_wavefront(fold3d_ctx *c, const fold3d_grid &g, const fold3d_med
     WaveArgs a;
     memset(&a, 0, sizeof a);
     a.flags = c->w_flags;
+    a.fshift = c->w_fshift;
     a.work = c->w_counters;
     a.status = c->w_counters + 1;
     a.maxd = c->d_maxd;
@@ -1600,6 +1604,7 @@ int fold3d_selftest_wait_timeout(fold3d_ctx *c, double timeout_ms)
     WaveArgs a;
     memset(&a, 0, sizeof a);
     a.flags = c->w_flags;
+    a.fshift = c->w_fshift;
     a.work = c->w_counters;
     a.status = c->w_counters + 1;
     a.maxd = c->d_maxd;

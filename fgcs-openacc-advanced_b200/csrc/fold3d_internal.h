@@ -98,6 +98,13 @@ enum Variant {
 #endif
 constexpr unsigned kPollNs = FOLD3D_POLL_NS;
 
+// Passes of at most this many items have a 32-byte sector for each completion
+// flag (128 MB at most): the many waiting warps and CTAs poll a step's few
+// flags, and 32 of them in one line are served one after another.  ms, 4 and 32
+// bytes per flag: drift 256^3, 8 sweeps from the host 128, 116; float32 TTI
+// 380x319x257 69.7, 63.9; 512^3 346, 347 (more flags than this).
+constexpr long long kSpreadFlags = 1ll << 22;
+
 // Items a batched pass's CTA claims at a time (1..32); build option.  24
 // instances of 96 to 200 points per axis to 1e-10, for 1, 2, 4 and 8: 297, 274,
 // 327, 498 ms: fewer, and every item pays for the claim and the instance; more,
@@ -161,7 +168,8 @@ struct WaveArgs {
     unsigned epoch;              // number of this pass (monotonic per context)
     unsigned skip_from;          // passes numbered below this never skip
     unsigned long long timeout_ns;
-    unsigned *flags;             // [steps][tiles]: pass number when the item finished
+    unsigned *flags;             // [steps][tiles]: pass number when the item finished, 1 << fshift words apart
+    int fshift;
     // change maps, [plane 0..n+1][tile]: the last pass a point changed; of this
     // pass's orientation, and of those with normal axes ua and va
     unsigned *mod[3];

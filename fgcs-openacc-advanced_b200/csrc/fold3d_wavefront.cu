@@ -166,7 +166,7 @@ __device__ __forceinline__ bool wave_item(R *__restrict__ T, const WaveArgs &a,
             const int nt = nv * a.ntu + nu;
             if (may_skip) recent = (__ldcg(a.mod[0] + (long long)src * ntiles + nt) + 5u >= a.epoch);
             if (p > 0) {
-                const unsigned f = wait_flag(a.flags + (long long)(p - 1) * ntiles + nt, want, a.status, a.timeout_ns);
+                const unsigned f = wait_flag(a.flags + (((long long)(p - 1) * ntiles + nt) << a.fshift), want, a.status, a.timeout_ns);
                 timed_out = f == 0;
                 recent |= (int)(f & 1u);
             }
@@ -190,7 +190,7 @@ __device__ __forceinline__ bool wave_item(R *__restrict__ T, const WaveArgs &a,
     // publish: the barrier makes every thread's stores precede thread 0's
     // release store, which orders them (cumulatively) before the flag
     __syncthreads();
-    if (tid == 0) st_release(a.flags + item, want | (unsigned)changed);
+    if (tid == 0) st_release(a.flags + ((long long)item << a.fshift), want | (unsigned)changed);
     return true;
 }
 
@@ -244,7 +244,7 @@ template <int TV, class Rows> __device__ __forceinline__ void warp_items(const W
         const int nu = tu + lane % 3 - 1, nv = tv + lane / 3 - 1, nt = nv * a.ntu + nu;
         const bool in = lane < 9 && nu >= 0 && nu < a.ntu && nv >= 0 && nv < a.ntv;
         recent = in && may_skip && __ldcg(a.mod[0] + (long long)(a.first_src + p * a.sg) * ntiles + nt) + 5u >= a.epoch;
-        return (in && p > 0) ? a.flags + (long long)(p - 1) * ntiles + nt : nullptr;
+        return (in && p > 0) ? a.flags + (((long long)(p - 1) * ntiles + nt) << a.fshift) : nullptr;
     };
     // The warp holds two claimed items: the flags of the second are read while
     // the first is worked on, and the fence that publishes the first also
@@ -290,7 +290,7 @@ template <int TV, class Rows> __device__ __forceinline__ void warp_items(const W
             prefetch();
         }
         fenced = !skip;
-        if (lane == 0) st_relaxed(a.flags + item, want | any);
+        if (lane == 0) st_relaxed(a.flags + ((long long)item << a.fshift), want | any);
         __syncwarp();
         if (changed) {
             wave_mark<1, TV>(a, u, v0, tgt);
@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(kWaveThreads, wave_min_blocks<double>())
                 if (may_skip) recent = __ldcg(a.mod[0] + (long long)src * ntiles + nt) + 5u >= a.epoch;
                 if (p > 0) {
                     const unsigned f =
-                        wait_flag(a.flags + (long long)(p - 1) * ntiles + nt, want, a.status, a.timeout_ns);
+                        wait_flag(a.flags + (((long long)(p - 1) * ntiles + nt) << a.fshift), want, a.status, a.timeout_ns);
                     gave_up = f == 0;
                     recent |= f & 1u;
                 }
@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(kWaveThreads, wave_min_blocks<double>())
         if (claims) s_item[slot ^ 1] = (claim < total) ? (int)claim : -1;
         const bool any = __syncthreads_or(changed);  // precedes the release: every thread's stores come before the flag
         if (threadIdx.x == 32) {
-            st_release(a.flags + item, want | (any ? 1u : 0u));
+            st_release(a.flags + ((long long)item << a.fshift), want | (any ? 1u : 0u));
             if (any) a.mod[0][(long long)tgt * ntiles + t] = a.epoch;
         }
     }
