@@ -218,8 +218,8 @@ __device__ __forceinline__ bool adj_item(const AdjWaveArgs &b, const EllipParam 
         // in the queue and never publish (nor push)
         if (nu >= 0 && nu < a.ntu && nv >= 0 && nv < a.ntv &&
             b.has[(long long)(tgt + a.sg) * ntiles + nv * a.ntu + nu]) {
-            timed_out = wait_flag(a.flags + (long long)(p - 1) * ntiles + nv * a.ntu + nu, want, a.status,
-                                  a.timeout_ns) == 0;
+            timed_out = wait_flag(a.flags + (((long long)(p - 1) * ntiles + nv * a.ntu + nu) << a.fshift), want,
+                                  a.status, a.timeout_ns) == 0;
         }
     }
     if (__syncthreads_or(timed_out)) return false;
@@ -238,7 +238,7 @@ __device__ __forceinline__ bool adj_item(const AdjWaveArgs &b, const EllipParam 
     // publish: the barrier makes every thread's atomics precede thread 0's
     // release store, which orders them (cumulatively) before the flag
     __syncthreads();
-    if (tid == 0) st_release(a.flags + item, want);
+    if (tid == 0) st_release(a.flags + ((long long)item << a.fshift), want);
     return true;
 }
 

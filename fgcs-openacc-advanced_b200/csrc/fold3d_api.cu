@@ -188,6 +188,7 @@ struct fold3d_ctx {
     std::vector<int> bkey;                   // dims of the instances the scratch is sized for
     unsigned *b_scratch = nullptr;           // flags and change maps of all instances
     std::vector<size_t> b_flag_off, b_mod_off[3];
+    int b_fshift = 0;                        // log2 of the words between two flags
     unsigned long long *b_slots = nullptr;   // [2n]: max|dT| and evaluated points per instance
     unsigned *b_counters = nullptr;          // work, status
     double *adj_pushed = nullptr;            // adjoint: lambda already pushed, per cell
@@ -649,6 +650,19 @@ static int batch_scratch(fold3d_ctx *c, const std::vector<fold3d_grid> &grids, i
     int max_steps = 0;
     c->b_flag_off.assign(n, 0);
     for (int b = 0; b < 3; ++b) c->b_mod_off[b].assign(n, 0);
+    long long flags = 0;  // of the pass with the most of them, per instance
+    for (int i = 0; i < n; ++i) {
+        const fold3d_grid &g = grids[i];
+        const int dims[3] = {g.nx, g.ny, g.nz};
+        long long most = 0;
+        for (int b = 0; b < 3; ++b) {
+            int ntu, ntv;
+            orient_tiles(g, b, ntu, ntv, tv);
+            most = std::max(most, (long long)(dims[b] - 1) * ntu * ntv);
+        }
+        flags += most;
+    }
+    c->b_fshift = flags <= kSpreadFlags ? 3 : 0;
     for (int i = 0; i < n; ++i) {
         const fold3d_grid &g = grids[i];
         const int dims[3] = {g.nx, g.ny, g.nz};
@@ -662,7 +676,7 @@ static int batch_scratch(fold3d_ctx *c, const std::vector<fold3d_grid> &grids, i
             max_steps = std::max(max_steps, dims[b] - 1);
         }
         c->b_flag_off[i] = words;
-        words += fw;
+        words += fw << c->b_fshift;
     }
     cudaError_t e;
     if ((e = cudaMalloc(&c->b_scratch, words * 4)) != cudaSuccess ||
@@ -818,6 +832,7 @@ static int solve_batch_cfg(fold3d_ctx *c, int n, const SolveInst *in, bool f32, 
             a.first_src = pass_first(a.pg, dir);
             a.timeout_ns = 4000000000ull;
             a.flags = c->b_scratch + c->b_flag_off[i];
+            a.fshift = c->b_fshift;
             unsigned *const maps[3] = {c->b_scratch + c->b_mod_off[0][i], c->b_scratch + c->b_mod_off[1][i],
                                        c->b_scratch + c->b_mod_off[2][i]};
             pass_maps(a, g, maps, tv);
@@ -1242,6 +1257,7 @@ static int adjoint_batch(fold3d_ctx *c, int n, const AdjInst *in, bool f32, int 
                 a.first_src = pass_first(a.pg, dir) + d.sg * pass_count(a.pg);  // the forward pass's last target
                 a.timeout_ns = 4000000000ull;
                 a.flags = c->b_scratch + c->b_flag_off[i];
+                a.fshift = c->b_fshift;
                 a.work = c->b_counters;
                 a.status = c->b_counters + 1;
                 a.maxd = c->b_slots + i;
