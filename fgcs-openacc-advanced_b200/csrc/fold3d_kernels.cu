@@ -39,33 +39,49 @@ __device__ __forceinline__ void block_max_to(double d, unsigned long long *out)
 }
 
 // The nine previous-plane magnitudes around the target whose source point
-// is `src` (the source plane is not written by the launch: read-only path).
+// is `src`.  The source plane is not written by the launch: RO reads it through
+// the read-only path, which a launch that may begin before the last plane's has
+// ended must not.
 struct Nbr9 {
     double st, xt, yt, xnt, ynt, txy, txm, tym, txnyn;
 };
-__device__ __forceinline__ Nbr9 load_nbr(const double *__restrict__ T, long long src, const PlaneGeom &g)
+template <bool RO> __device__ __forceinline__ double load_src(const double *p) { return RO ? __ldg(p) : *p; }
+template <bool RO = true>
+__device__ __forceinline__ Nbr9 load_nbr(const double *T, long long src, const PlaneGeom &g)
 {
     Nbr9 s;
-    s.st = fabs(__ldg(T + src));
-    s.xt = fabs(__ldg(T + src + g.sx));
-    s.yt = fabs(__ldg(T + src + g.sy));
-    s.xnt = fabs(__ldg(T + src - g.sx));
-    s.ynt = fabs(__ldg(T + src - g.sy));
-    s.txm = fabs(__ldg(T + src + g.sx - g.sy));
-    s.txy = fabs(__ldg(T + src + g.sx + g.sy));
-    s.tym = fabs(__ldg(T + src - g.sx + g.sy));
-    s.txnyn = fabs(__ldg(T + src - g.sx - g.sy));
+    s.st = fabs(load_src<RO>(T + src));
+    s.xt = fabs(load_src<RO>(T + src + g.sx));
+    s.yt = fabs(load_src<RO>(T + src + g.sy));
+    s.xnt = fabs(load_src<RO>(T + src - g.sx));
+    s.ynt = fabs(load_src<RO>(T + src - g.sy));
+    s.txm = fabs(load_src<RO>(T + src + g.sx - g.sy));
+    s.txy = fabs(load_src<RO>(T + src + g.sx + g.sy));
+    s.tym = fabs(load_src<RO>(T + src - g.sx + g.sy));
+    s.txnyn = fabs(load_src<RO>(T + src - g.sx - g.sy));
     return s;
 }
 
-__global__ void __launch_bounds__(256) plane_kernel_fast(double *__restrict__ T, long long src_off, PlaneGeom g,
+// The default form.  A sweep is one launch per plane, each depending on the
+// last, and a plane of 128^2 points is 64 blocks: what bounds it is one point's
+// chain of operations and the gap between launches.  The launch may begin while
+// the last plane's is still running (programmatic dependent launch), copies its
+// table meanwhile, and waits before it touches the field.  A sweep of plane
+// calls at 128^3: 13.3 ms with FP64 gates, 10.2 with the float filter, 9.1 so;
+// 256^3, 4 sweeps: 95 -> 81.
+__global__ void __launch_bounds__(256) plane_kernel_fast(double *T, long long src_off, PlaneGeom g,
                                                          const __grid_constant__ DirTable tab,
-                                                         unsigned long long *__restrict__ maxd)
+                                                         unsigned long long *maxd)
 {
     __shared__ double s_fan[9][256];
     __shared__ float s_dif[9][256];
     __shared__ DirTable s_tab;
     const int tid = threadIdx.x + 32 * threadIdx.y;
+    // The next plane's launch may set itself up from here on; this one waits
+    // for the plane before it once its own table is in place.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    copy_table(s_tab, tab, tid, 256);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int u = blockIdx.x * 32 + threadIdx.x + 1;
     const int v = blockIdx.y * 8 + threadIdx.y + 1;
     const bool active = u <= g.nu && v <= g.nv;
@@ -74,13 +90,12 @@ __global__ void __launch_bounds__(256) plane_kernel_fast(double *__restrict__ T,
     if (active) {
         const long long src = src_off + (long long)u * g.su + (long long)v * g.sv;
         tgt = src + g.sn;
-        const Nbr9 s = load_nbr(T, src, g);
+        const Nbr9 s = load_nbr<false>(T, src, g);
         const double got[9] = {s.xt, s.txy, s.yt, s.tym, s.xnt, s.txnyn, s.ynt, s.txm, s.st};
 #pragma unroll
         for (int r = 0; r < 9; ++r) fan[r] = got[r];
         told = T[tgt];
     }
-    copy_table(s_tab, tab, tid, 256);
     __syncthreads();
     const double tnew = point_update_fan(active, told, fan, s_tab, &s_fan[0][tid], &s_dif[0][tid], 256);
     if (active) T[tgt] = tnew;
@@ -288,7 +303,16 @@ cudaError_t launch_plane(double *T, const PlaneGeom &pg, const LocalFrameH &Lh, 
         plane_kernel_literal<<<grid, block, 0, s>>>(T, off, pg, L, maxd);
     } else {
         if (!tab) return cudaErrorInvalidValue;
-        plane_kernel_fast<<<grid, block, 0, s>>>(T, off, pg, *tab, maxd);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = grid;
+        cfg.blockDim = block;
+        cfg.stream = s;
+        cudaLaunchAttribute at = {};
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, plane_kernel_fast, T, off, pg, *tab, maxd);
     }
     return cudaGetLastError();
 }
