@@ -503,7 +503,19 @@ static int drift_tile_rows(const fold3d_grid &g)
 {
     if (FOLD3D_DRIFT_TV) return FOLD3D_DRIFT_TV;
     const double rows = 3.0 * g.nx * g.ny * g.nz / 32.0 / ((double)g.nx + g.ny + g.nz);
-    return rows < 12000.0 ? 1 : rows < 32000.0 ? 2 : 4;
+    int tv = rows < 12000.0 ? 1 : rows < 32000.0 ? 2 : 4;
+    // flat grids fill few of a row's 32 points: no more than 32 M items (flags
+    // and map words) for their sake
+    const int n[3] = {g.nx, g.ny, g.nz};
+    for (int b = 0; b < 3 && tv < 4; ++b) {
+        int ntu, ntv;
+        orient_tiles(g, b, ntu, ntv, tv);
+        if ((double)n[b] * ntu * ntv > 33554432.0) {
+            tv *= 2;
+            b = -1;
+        }
+    }
+    return tv;
 }
 
 // T: double, or float when f32 (elliptical medium only).

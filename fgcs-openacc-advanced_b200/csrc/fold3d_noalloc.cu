@@ -136,7 +136,7 @@ int solve_noalloc(const fold3d_grid *g, const fold3d_medium *m, double *T, const
 
     const auto t0 = std::chrono::steady_clock::now();
     cudaStream_t s = (cudaStream_t)stream;
-    DirTable tab;  // one direction's constants at a time (4.6 KiB of host stack)
+    DirTable tab;  // one direction's constants at a time (7 KiB of host stack)
     int sweeps = 0;
     unsigned long long bits = 0;
     while (sweeps < o->max_sweeps) {
