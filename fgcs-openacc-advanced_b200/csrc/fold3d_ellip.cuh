@@ -31,6 +31,9 @@
 // (their square roots are well conditioned there), in float as in double;
 // with B = 0 (a rounded Schur complement <= 0) the gates are the plain ones.
 //
+// Those gates serve float fields; double fields are updated behind a float
+// filter instead (ell_update_fan, below).
+//
 // oracle/fold3d_oracle.c (orc_ell_*) states the same computation on the
 // CPU; this file follows it operation by operation (no FMA contraction), so
 // the two agree bit for bit.
@@ -341,6 +344,12 @@ __host__ __device__ __forceinline__ R point_update_ellip(R told, R st, const R n
 //
 // float32 fields do not take this path: their times are rounded to 1e-7 of
 // their own size, so candidates that the filter tells apart often tie.
+//
+// ms before (gated FP64 candidates) and now, with the passes' other changes of
+// the time (waits, barriers, batch chunks): TTI 512^3 to 1e-10 374, 248; 24
+// instances of 96 to 200 points per axis 476, 264; 8 sources at 192^3 with their gradients 471,
+// 249; 128^3 14.3, 12.5.  A point now costs 0.3 to 0.4 FP64 candidates of the
+// 33; what bounds a pass is in fold3d_wavefront.cu.
 // ---------------------------------------------------------------------------
 __host__ __device__ __forceinline__ float ell_rsqrt(float x)
 {

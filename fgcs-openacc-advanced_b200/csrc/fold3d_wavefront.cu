@@ -310,13 +310,13 @@ template <int TV, class Rows> __device__ __forceinline__ void warp_items(const W
 // three new ones read while the last row is worked on.
 //
 // What bounds it: the latency of a point's update and of the exchange between
-// plane steps, not bytes (10 DRAM bytes per update) and not issue (47% of the
-// cycles at 1280^2 planes).  Per row of 32 points it runs 520 warp instructions
-// (about 930 before the float filter).  In a settled field (no tile skipped)
+// plane steps, not bytes (10 DRAM bytes per update) and not issue alone (59% of the
+// cycles at 1280^2 planes).  Per row of 32 points it runs 450 to 940 warp
+// instructions (930 to 1360 before the float filter).  In a settled field (no tile skipped)
 // a plane step takes 6.6, 9.6, 12.6 and 61 us at 64, 256, 512 and 1280 points
 // per axis, of which the claims, waits and publishing alone 2.5, 4.0, 5.7 and 9.
-// ms before (a CTA per 32 x 4 tile, FP64 gates) and now: 64^3, 8 sweeps 36 ->
-// 20; 512^3, 8 sweeps 455 -> 335; 1280^3, 2 sweeps 1515 -> 1126.
+// ms before (a CTA per 32 x 4 tile, FP64 gates) and now: 64^3, 8 sweeps 36.8 ->
+// 19.4; 512^3, 8 sweeps 453 -> 350; 1280^3, 2 sweeps 1518 -> 1135.
 template <int TV>
 __global__ void __launch_bounds__(kWaveThreads, FOLD3D_WAVE_MINB_DRIFT)
     drift_pass_kernel(double *__restrict__ T, WaveArgs a, const __grid_constant__ DirTable tab)
@@ -388,7 +388,9 @@ __global__ void __launch_bounds__(kWaveThreads, FOLD3D_WAVE_MINB_DRIFT)
 // others go on.  On smaller planes, and for float fields, the plane-to-plane
 // chain binds and wave_item_kernel is faster, where thread 0 publishes before
 // anything of the next item begins (ms; two barriers, this: 128^3 to 1e-10
-// 12.7, 12.2; 512^3 312, 339; float32 380x319x257 72.4, 69.8).
+// 12.7, 12.2; 512^3 312, 339; float32 380x319x257 72.4, 69.8).  What bounds
+// both is the chain from step to step, and on x-normal planes loads of which
+// every lane's is a sector of its own (2 to 3 times a k pass at 512^3).
 template <class R>
 __global__ void __launch_bounds__(kWaveThreads, wave_min_blocks<R>())
     wave_item_kernel(R *__restrict__ T, WaveArgs a, const __grid_constant__ EllipParam tab)
