@@ -900,6 +900,12 @@ static int solve_batch_cfg(fold3d_ctx *c, int n, const SolveInst *in, bool f32, 
     ctl.status = c->b_counters + 1;
     // a grid as large as the biggest pass can use (instances drop out later)
     const int grid = (int)std::min<long long>(max_total, (long long)c->sms * bps);
+    for (int dir = 0; dir < 6; ++dir) {
+        long long tiles = 0;  // of one plane step of the whole batch
+        const BatchStage h = batch_stage(c, c->b_stage_h, dir, n);
+        for (int q = 0; q < n; ++q) tiles += h.tiles[q];
+        args[dir].chunk = tiles >= (long long)kBatchBusy * grid ? kBatchChunk : 2;
+    }
 
     // the graph: prologue (tables), then while (more) { six passes; restage }
     cudaGraph_t graph = nullptr;

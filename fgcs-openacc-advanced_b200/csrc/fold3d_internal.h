@@ -105,14 +105,14 @@ constexpr unsigned kPollNs = FOLD3D_POLL_NS;
 // 380x319x257 69.7, 63.9; 512^3 346, 347 (more flags than this).
 constexpr long long kSpreadFlags = 1ll << 22;
 
-// Items a batched pass's CTA claims at a time (1..32); build option.  24
-// instances of 96 to 200 points per axis to 1e-10, for 1, 2, 4 and 8: 297, 274,
-// 327, 498 ms: fewer, and every item pays for the claim and the instance; more,
-// and items that others wait for stand in a queue.
-#ifndef FOLD3D_BATCH_CHUNK
-#define FOLD3D_BATCH_CHUNK 2
-#endif
-constexpr int kBatchChunk = FOLD3D_BATCH_CHUNK;
+// Items a batched pass's CTA claims at a time: two, or four when a plane step of
+// the batch has kBatchBusy tiles or more for every resident CTA.  Few, and every
+// item pays for the claim and the search for its instance; many, and items that
+// others wait for stand in a queue.  ms to 1e-10 in chunks of 2, 4 and 8: 24
+// instances of 96 to 200 points per axis (6 tiles per CTA) 274, 327, 498; 48 of
+// 96 to 256 (17) 832, 785, 927; 128 of them (46) 2202, 1972, 2070.
+constexpr int kBatchChunk = 4;
+constexpr int kBatchBusy = 10;
 static_assert(kBatchChunk >= 1 && kBatchChunk <= 32, "batch chunk");
 
 // Rows of the drift medium's tiles; build option, 0: by grid size
@@ -258,6 +258,7 @@ struct BatchArgs {
     int max_steps, dir;
     unsigned *work, *status;
     unsigned skip_from;           // first pass that may skip
+    int chunk;                    // items claimed at a time, at most kBatchChunk
 };
 // tv: tile height of the batch (2, 4 or 8 rows; 32 * tv threads per CTA).
 cudaError_t launch_batch_pass(const BatchArgs &b, bool f32, int tv, int grid, cudaStream_t s);

@@ -509,7 +509,7 @@ template <class R, int TV> constexpr int batch_min_blocks()
 template <class R, int TV>
 __global__ void __launch_bounds__(32 * TV, batch_min_blocks<R, TV>()) batch_pass_kernel(BatchArgs b)
 {
-    // A CTA claims kBatchChunk consecutive items at a time, and the first
+    // A CTA claims b.chunk consecutive items at a time, and the first
     // lanes of warp 0 locate them in parallel (two binary searches each over
     // the launch's tables): consecutive items mostly belong to one instance
     // (its tiles of a step come together), so the instance is staged once for
@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(32 * TV, batch_min_blocks<R, TV>()) batch_pass
     __shared__ double s_fan[sizeof(R) == 8 ? 9 * 32 * TV : 1];
     const unsigned total = *b.total;
     if (threadIdx.x == 0) {
-        const unsigned w = atomicAdd(b.work, (unsigned)kBatchChunk);
+        const unsigned w = atomicAdd(b.work, (unsigned)b.chunk);
         s_next = (w < total) ? (int)w : -1;
         s_n = 0;
         s_cur = -1;
@@ -540,12 +540,12 @@ __global__ void __launch_bounds__(32 * TV, batch_min_blocks<R, TV>()) batch_pass
             if (c0 < 0) break;
             __syncthreads();  // every thread has read s_n and s_next
             if (threadIdx.x < 32) {
-                const int n = (int)min((unsigned)kBatchChunk, total - (unsigned)c0);
+                const int n = (int)min((unsigned)b.chunk, total - (unsigned)c0);
                 if ((int)threadIdx.x < n)
                     batch_locate(b.step_off, b.step_k, b.tile_pre, b.max_steps, c0 + (int)threadIdx.x,
                                  s_loc[threadIdx.x][0], s_loc[threadIdx.x][1]);
                 if (threadIdx.x == 0) {
-                    const unsigned w = atomicAdd(b.work, (unsigned)kBatchChunk);
+                    const unsigned w = atomicAdd(b.work, (unsigned)b.chunk);
                     s_next = (w < total) ? (int)w : -1;
                     s_n = n;
                 }
