@@ -339,6 +339,19 @@ __host__ __device__ __forceinline__ R point_update_ellip(R told, R st, const R n
 // within 1e4 of sqrt(A.xx), sqrt(A.yy) of each other (their differences are off
 // by 1e-3 of those); it takes s off by up to 1e-3 (1 + s) and u by 0.01 plus
 // 1e-4 n |h|, in units of the spacings.  Elsewhere every candidate is kept.
+//
+// The tests tell the candidates' exact values apart, the update the rounded
+// ones.  What the margin of u (0.01 of a weight, so 0.007 of a spacing) keeps
+// out is above the smallest value by at least 2.5e-5 times f's curvature, which
+// for a u inside is at least 0.007 min(A.xx, A.yy, r) / sqrt(r) within the
+// limits above; a candidate is rounded to 4 ulp of T, the smaller of st and the
+// time.  So the tests are used up to T sqrt(r) = 2^26 min(A.xx, A.yy, r): 2^26
+// cell times where the spacings are alike, and less than half of where they
+// could disagree (with point sources the first differing records came at 1e11).
+// Beyond it, which takes a source on an absolute clock, the gates of
+// point_update_ellip choose: a candidate's rounded value is at least its
+// smallest source plus sqrt(r), rounded.
+//
 // What is kept runs through the FP64 candidates in the order of their ids, each
 // lane its own list, so the time and the winner are the same bits.
 //
@@ -385,6 +398,30 @@ __host__ __device__ __forceinline__ int ell_low(unsigned m)
     return __ffs((int)m) - 1;
 #else
     return __builtin_ctz(m);
+#endif
+}
+
+// The biased exponent of x.
+__host__ __device__ __forceinline__ unsigned ell_exp(double x)
+{
+#ifdef __CUDA_ARCH__
+    return ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
+#else
+    unsigned long long b;
+    __builtin_memcpy(&b, &x, sizeof b);
+    return (unsigned)(b >> 52) & 0x7ffu;
+#endif
+}
+// log2(a / b) of positive floats, off by less than one.
+__host__ __device__ __forceinline__ int ell_log2(float a, float b)
+{
+#ifdef __CUDA_ARCH__
+    return (__float_as_int(a) - __float_as_int(b)) >> 23;
+#else
+    int x, y;
+    __builtin_memcpy(&x, &a, sizeof x);
+    __builtin_memcpy(&y, &b, sizeof y);
+    return (x - y) >> 23;
 #endif
 }
 
@@ -470,30 +507,36 @@ __host__ __device__ __forceinline__ EllipA ell_local_v(int kind, const EllipDir 
 // rim edge and triangle; bit 8 of vert, st.
 struct EllKeep {
     unsigned vert, spoke, rim, tri;
-    float Eb;  // above the new time's distance from st, +inf if unknown
+    // above the new time's distance from st; where all are kept, +inf, or -inf
+    // for times too large to judge
+    float Eb;
 };
 
-// c: float(st - s_r) of the rim, E: float(tn - st).
-__host__ __device__ __forceinline__ EllKeep ell_filter(bool active, const float c[8], float E, const EllipAT<float> &A)
+// c: float(st - s_r) of the rim, E: float(tn - st), eT: the exponent (ell_exp)
+// of the smaller of st and tn.
+__host__ __device__ __forceinline__ EllKeep ell_filter(bool active, const float c[8], float E, unsigned eT,
+                                                       const EllipAT<float> &A)
 {
     EllKeep K = {0u, 0u, 0u, 0u, HUGE_VALF};
     const float cof = A.xx * A.yy - A.xy * A.xy, icof = ell_rcp(cof);
     const float px = (A.yy * A.xz - A.xy * A.yz) * icof, py = (A.xx * A.yz - A.xy * A.xz) * icof;
     const float r = A.zz - (A.xz * px + A.yz * py);
     const float big = fmaxf(A.xx, A.yy), small = fminf(A.xx, A.yy);
-    // every comparison is false for a NaN
-    const bool sane = small > 1e-30f && big < 1e30f && A.zz < 1e30f && cof > 0.25f * (A.xx * A.yy) &&
-                      r > 0.25f * A.zz && r > 1e-3f * big && E > -1e30f;
     float mx = 0.0f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) mx = fmaxf(mx, c[k]);
+    // every comparison is false for a NaN
+    const bool sane = small > 1e-30f && big < 1e30f && A.zz < 1e30f && cof > 0.25f * (A.xx * A.yy) &&
+                      r > 0.25f * A.zz && r > 1e-3f * big && E > -1e30f;
     float Eb = fmaf(fabsf(E), 1e-6f, E);  // above the new time's distance from st
     const float sr = r * ell_rsqrt(fmaxf(r, 1e-36f));
     const float far2 = 1e8f * small;
     const bool near = active && (!sane || Eb + mx > 0.99f * sr);
     if (!ell_any(near)) return K;
+    // T above 2^26 min(small, r) / sr, to a factor of two
+    const bool coarse = sane && (int)eT - 1023 > 25 + ell_log2(fminf(small, r), sr);
+    const bool go = near && sane && !coarse;
     unsigned VA = 0, VB = 0, VC = 0, TR = 0;
-    const bool go = near && sane;
     // ||X - p|| is at least this on the fan's sides x = 1, y = 1, x = -1, y = -1
     const float kx = cof * ell_rcp(A.yy), ky = cof * ell_rcp(A.xx);
     float side[4];
@@ -554,7 +597,7 @@ __host__ __device__ __forceinline__ EllKeep ell_filter(bool active, const float 
     }
     K.vert = ((VA | VC) & prev(VB | VC) & early) | (((VA | VB) == 0xffu) ? 0x100u : 0u);
     K.Eb = Eb;
-    if (near && !sane) K = {0x1ffu, 0xffu, 0xffu, 0xffu, HUGE_VALF};
+    if (near && !go) K = {0x1ffu, 0xffu, 0xffu, 0xffu, coarse ? -HUGE_VALF : HUGE_VALF};
     return K;
 }
 
@@ -590,16 +633,6 @@ __host__ __device__ __forceinline__ bool ell_vertex_may(const EllipAT<float> &A,
 
 // x / c from r = RN(1/c) where that is exact (Markstein's two remainder
 // corrections, as div_by_const in fold3d_fast.cuh), else x / c.
-__host__ __device__ __forceinline__ unsigned ell_exp(double x)
-{
-#ifdef __CUDA_ARCH__
-    return ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
-#else
-    unsigned long long b;
-    __builtin_memcpy(&b, &x, sizeof b);
-    return (unsigned)(b >> 52) & 0x7ffu;
-#endif
-}
 __host__ __device__ __forceinline__ double ell_div(double x, double c, double r, bool ok)
 {
     if (!ok || ell_exp(x) - (1023u - 400u) > 800u) return x / c;
@@ -690,9 +723,24 @@ __host__ __device__ __forceinline__ double ell_update_fan(bool active, double to
     }
     sh[8 * stride] = st;
     const EllipAT<float> Af = ell_local_f(kind, D, v);
-    const EllKeep K = ell_filter(active, c, (float)(tn - st), Af);
+    EllKeep K = ell_filter(active, c, (float)(tn - st), ell_exp(tn < st ? tn : st), Af);
     if (ell_any((K.vert | K.spoke | K.rim | K.tri) != 0)) {
-        const bool known = K.Eb < HUGE_VALF;
+        const bool known = fabsf(K.Eb) < HUGE_VALF;
+        const bool gates = K.Eb == -HUGE_VALF;
+        if (ell_any(gates)) {  // point_update_ellip's tests in place of the filter's
+            if (gates) {
+                const EllipA A = ell_local_v(kind, D, v);
+                const double g = ell_skip_bound(A);
+#pragma unroll 1
+                for (int r = 0; r < 8; ++r) {
+                    const double a = sh[r * stride], b = ell_min(a, sh[((r + 1) & 7) * stride]);
+                    if (tn <= a + g) K.vert &= ~(1u << r);
+                    if (tn <= ell_min(st, a) + g) K.spoke &= ~(1u << r);
+                    if (tn <= b + g) K.rim &= ~(1u << r);
+                    if (tn <= ell_min(st, b) + g) K.tri &= ~(1u << r);
+                }
+            }
+        }
         unsigned vert = K.vert & 0xffu, edge = 0;
         for (unsigned m = vert; ell_any(m != 0);) {
             if (m) {
