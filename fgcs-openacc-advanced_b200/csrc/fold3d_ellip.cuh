@@ -339,6 +339,8 @@ __host__ __device__ __forceinline__ R point_update_ellip(R told, R st, const R n
 // within 1e4 of sqrt(A.xx), sqrt(A.yy) of each other (their differences are off
 // by 1e-3 of those); it takes s off by up to 1e-3 (1 + s) and u by 0.01 plus
 // 1e-4 n |h|, in units of the spacings.  Elsewhere every candidate is kept.
+// Where a source is NaN the tests of point_update_ellip decide, for their order
+// does.
 //
 // The tests tell the candidates' exact values apart, the update the rounded
 // ones.  What the margin of u (0.01 of a weight, so 0.007 of a spacing) keeps
@@ -508,9 +510,21 @@ __host__ __device__ __forceinline__ EllipA ell_local_v(int kind, const EllipDir 
 struct EllKeep {
     unsigned vert, spoke, rim, tri;
     // above the new time's distance from st; where all are kept, +inf, or -inf
-    // for times too large to judge
+    // for times too large to judge, or NaN for a NaN among the sources
     float Eb;
 };
+
+// The largest; NaN if one of them is.
+__host__ __device__ __forceinline__ float ell_max_nan(float a, float b, float c)
+{
+#ifdef __CUDA_ARCH__
+    float y;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+    return y;
+#else
+    return a != a ? a : b != b ? b : c != c ? c : fmaxf(fmaxf(a, b), c);
+#endif
+}
 
 // c: float(st - s_r) of the rim, E: float(tn - st), eT: the exponent (ell_exp)
 // of the smaller of st and tn.
@@ -524,10 +538,10 @@ __host__ __device__ __forceinline__ EllKeep ell_filter(bool active, const float 
     const float big = fmaxf(A.xx, A.yy), small = fminf(A.xx, A.yy);
     float mx = 0.0f;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) mx = fmaxf(mx, c[k]);
+    for (int k = 0; k < 8; k += 2) mx = ell_max_nan(mx, c[k], c[k + 1]);
     // every comparison is false for a NaN
     const bool sane = small > 1e-30f && big < 1e30f && A.zz < 1e30f && cof > 0.25f * (A.xx * A.yy) &&
-                      r > 0.25f * A.zz && r > 1e-3f * big && E > -1e30f;
+                      r > 0.25f * A.zz && r > 1e-3f * big && E > -1e30f && mx < 1e30f;
     float Eb = fmaf(fabsf(E), 1e-6f, E);  // above the new time's distance from st
     const float sr = r * ell_rsqrt(fmaxf(r, 1e-36f));
     const float far2 = 1e8f * small;
@@ -597,7 +611,7 @@ __host__ __device__ __forceinline__ EllKeep ell_filter(bool active, const float 
     }
     K.vert = ((VA | VC) & prev(VB | VC) & early) | (((VA | VB) == 0xffu) ? 0x100u : 0u);
     K.Eb = Eb;
-    if (near && !go) K = {0x1ffu, 0xffu, 0xffu, 0xffu, coarse ? -HUGE_VALF : HUGE_VALF};
+    if (near && !go) K = {0x1ffu, 0xffu, 0xffu, 0xffu, coarse ? -HUGE_VALF : mx == mx ? HUGE_VALF : mx};
     return K;
 }
 
@@ -726,11 +740,17 @@ __host__ __device__ __forceinline__ double ell_update_fan(bool active, double to
     EllKeep K = ell_filter(active, c, (float)(tn - st), ell_exp(tn < st ? tn : st), Af);
     if (ell_any((K.vert | K.spoke | K.rim | K.tri) != 0)) {
         const bool known = fabsf(K.Eb) < HUGE_VALF;
-        const bool gates = K.Eb == -HUGE_VALF;
+        const bool gates = K.Eb != K.Eb || K.Eb == -HUGE_VALF;
         if (ell_any(gates)) {  // point_update_ellip's tests in place of the filter's
             if (gates) {
                 const EllipA A = ell_local_v(kind, D, v);
-                const double g = ell_skip_bound(A);
+                if (K.vert >> 8) ell_vertex(tn, win, 0, A, 0.0, st, 0, 0);
+                K.vert &= 0xffu;
+                double m = st;
+#pragma unroll 1
+                for (int r = 0; r < 8; ++r) m = ell_min(m, sh[r * stride]);
+                if (!(tn > m)) K.vert = K.spoke = K.rim = K.tri = 0;  // a NaN among the sources decides it, too
+                const double g = K.Eb == K.Eb ? ell_skip_bound(A) : 0.0;
 #pragma unroll 1
                 for (int r = 0; r < 8; ++r) {
                     const double a = sh[r * stride], b = ell_min(a, sh[((r + 1) & 7) * stride]);
