@@ -248,9 +248,8 @@ template <int TV, class Rows> __device__ __forceinline__ void warp_items(const W
     };
     // The warp holds two claimed items: the flags of the second are read while
     // the first is worked on, and the fence that publishes the first also
-    // orders that read before the second's loads.  A skipped item has written
-    // nothing, so its flag needs no fence (who waits for it reads what earlier
-    // passes left); the next item that is not skipped then fences first.
+    // orders that read before the second's loads (with the warp barrier after it,
+    // which carries the nine watching lanes' order to all lanes).
     unsigned ahead = 0;
     if (lane == 0) ahead = atomicAdd(a.work, 1u);
     unsigned item = __shfl_sync(0xffffffffu, ahead, 0);
@@ -259,7 +258,6 @@ template <int TV, class Rows> __device__ __forceinline__ void warp_items(const W
     bool recent = false;
     const unsigned *fl = item < total ? watch(item, p, t, tu, tv, recent) : nullptr;
     unsigned f = 0;
-    bool fenced = true;  // nothing has been read relaxed since the last fence
     while (item < total) {
         bool gave_up = false;
         if (fl && f < want) {
@@ -269,6 +267,7 @@ template <int TV, class Rows> __device__ __forceinline__ void warp_items(const W
         recent |= fl && (f & 1u);
         if (__any_sync(0xffffffffu, gave_up)) break;
         const bool skip = may_skip && !__any_sync(0xffffffffu, recent);
+        __syncwarp();  // the watching lanes' acquire comes before every lane's loads (votes order no memory)
         const unsigned next = __shfl_sync(0xffffffffu, ahead, 0);
         if (lane == 0) ahead = atomicAdd(a.work, 1u);
         const int src = a.first_src + p * a.sg, tgt = src + a.sg, u = tu * 32 + lane + 1, v0 = tv * TV + 1;
@@ -281,15 +280,13 @@ template <int TV, class Rows> __device__ __forceinline__ void warp_items(const W
         };
         unsigned changed = 0, any = 0;
         if (!skip) {
-            if (!fenced) fence_acq_rel();
             changed = rows(src, u, v0, min(TV, a.pg.nv - v0 + 1), u <= a.pg.nu, prefetch);
             any = __any_sync(0xffffffffu, changed != 0) ? 1u : 0u;
-            __syncwarp();
-            fence_acq_rel();
         } else {
             prefetch();
         }
-        fenced = !skip;
+        __syncwarp();
+        fence_acq_rel();
         if (lane == 0) st_relaxed(a.flags + ((long long)item << a.fshift), want | any);
         __syncwarp();
         if (changed) {
