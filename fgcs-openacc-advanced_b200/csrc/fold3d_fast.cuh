@@ -351,7 +351,7 @@ __host__ __device__ __forceinline__ unsigned push_sign(unsigned m, float x)
 #else
     uint32_t b;
     std::memcpy(&b, &x, sizeof b);
-    return (m << 1) | (b >> 31);
+    return (m << 1) | (x != x ? 0u : b >> 31);  // the device's NaN has a clear sign
 #endif
 }
 
@@ -490,7 +490,7 @@ __host__ __device__ __forceinline__ double point_update_fan(bool active, double 
     ch[8 * stride] = 0.0f;
     if (st < tn && f.d1_ok) tn = kmin(tn, st + f.K1);
     float E = (float)(tn - st);
-    const bool odd = !(E > -3e38f) || f.every;  // st infinite or beyond float, or a NaN: gate nothing
+    const bool odd = !(fabsf(E) < 3e38f) || f.every;  // a time infinite or beyond float, or a NaN: gate nothing
     const float mx = fmaxf(fmaxf(fmaxf(fmaxf(c[0], c[1]), fmaxf(c[2], c[3])), fmaxf(fmaxf(c[4], c[5]), fmaxf(c[6], c[7]))),
                            0.0f);
     if (lanes_any(active && (odd || fmaf(fabsf(E), 4e-7f, E) + mx > f.outer))) {
