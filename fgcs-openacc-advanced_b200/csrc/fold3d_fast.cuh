@@ -343,6 +343,18 @@ __host__ __device__ __forceinline__ float filter_rsqrt(float x)
 #endif
 }
 
+// The larger one; NaN if either is.
+__host__ __device__ __forceinline__ float max_nan(float a, float b)
+{
+#ifdef __CUDA_ARCH__
+    float y;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+    return y;
+#else
+    return a != a ? a : b != b ? b : fmaxf(a, b);
+#endif
+}
+
 // m with the sign bit of x appended.
 __host__ __device__ __forceinline__ unsigned push_sign(unsigned m, float x)
 {
@@ -498,8 +510,10 @@ __host__ __device__ __forceinline__ double point_update_fan(bool active, double 
         if (odd) mask = 0xffffffu;
         // the reference's early exit (:231), on the sources it names (not xnt
         // and ynt): a gate of its own, so judged in FP64 where float is unsure
-        const float lead = E + fmaxf(fmaxf(fmaxf(f.named[0] ? c[4] : c[0], f.named[1] == 2 ? c[2] : c[6]), fmaxf(c[1], c[7])),
-                                     fmaxf(c[5], c[3]));
+        // (NaN where one of them is NaN)
+        const float lead = E + max_nan(max_nan(max_nan(f.named[0] ? c[4] : c[0], f.named[1] == 2 ? c[2] : c[6]),
+                                               max_nan(c[1], c[7])),
+                                       max_nan(c[5], c[3]));
         const float unsure = 4e-7f * fabsf(E);
         if (tn < st && mask && !(lead > unsure)) {
             if (lead < -unsure || (tn < kmin(sh[f.named[0] * stride], sh[f.named[1] * stride]) &&

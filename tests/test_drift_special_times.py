@@ -35,7 +35,7 @@ def _same(orc, T, T0, h, F, a, what):
     assert np.array_equal(T.view(np.uint64)[~b], ref.view(np.uint64)[~b]), what
 
 
-KINDS = ["inf"]
+KINDS = ["inf", "nan"]
 
 
 @pytest.mark.parametrize("skip", [1, 2], ids=["searched", "closed-form"])
