@@ -426,7 +426,9 @@ static int reserve_passes(fold3d_ctx *c, unsigned passes)
     return FOLD3D_OK;
 }
 
-static int wave_scratch(fold3d_ctx *c, const fold3d_grid &g, int tv)
+// The clears run on the caller's stream, which need not wait for the legacy one,
+// and are over before the scratch counts as made.
+static int wave_scratch(fold3d_ctx *c, const fold3d_grid &g, int tv, cudaStream_t s)
 {
     if (c->w_flags && c->key_wg.nx == g.nx && c->key_wg.ny == g.ny && c->key_wg.nz == g.nz && c->key_wtv == tv)
         return FOLD3D_OK;
@@ -436,6 +438,7 @@ static int wave_scratch(fold3d_ctx *c, const fold3d_grid &g, int tv)
         c->w_mod[b] = nullptr;
     }
     c->w_flags = nullptr;
+    c->key_wg = fold3d_grid{};
     const int n[3] = {g.nx, g.ny, g.nz};
     size_t flag_words = 0;
     cudaError_t e;
@@ -445,13 +448,13 @@ static int wave_scratch(fold3d_ctx *c, const fold3d_grid &g, int tv)
         flag_words = std::max(flag_words, (size_t)(n[b] - 1) * ntu * ntv);
         const size_t words = (size_t)(n[b] + 2) * ntu * ntv;
         if ((e = cudaMalloc(&c->w_mod[b], words * 4)) != cudaSuccess ||
-            (e = cudaMemset(c->w_mod[b], 0, words * 4)) != cudaSuccess)
+            (e = cudaMemsetAsync(c->w_mod[b], 0, words * 4, s)) != cudaSuccess)
             return set_errorf(FOLD3D_ERR_NOMEM, "wavefront scratch: %s", cudaGetErrorString(e));
     }
     c->w_fshift = (long long)flag_words <= kSpreadFlags ? 3 : 0;
     flag_words <<= c->w_fshift;
     if ((e = cudaMalloc(&c->w_flags, flag_words * 4)) != cudaSuccess ||
-        (e = cudaMemset(c->w_flags, 0, flag_words * 4)) != cudaSuccess)
+        (e = cudaMemsetAsync(c->w_flags, 0, flag_words * 4, s)) != cudaSuccess)
         return set_errorf(FOLD3D_ERR_NOMEM, "wavefront scratch: %s", cudaGetErrorString(e));
     if (!c->w_counters) {
         if ((e = cudaMalloc(&c->w_counters, 2 * sizeof(unsigned))) != cudaSuccess ||
@@ -463,6 +466,7 @@ static int wave_scratch(fold3d_ctx *c, const fold3d_grid &g, int tv)
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, dev);
     }
+    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_error(e, "wavefront scratch");
     c->key_wtv = tv;
     c->key_wg = g;  // fresh flags and maps are zero, below every pass number to come
     return FOLD3D_OK;
@@ -526,7 +530,7 @@ static int solve_wavefront(fold3d_ctx *c, const fold3d_grid &g, const fold3d_med
     int rc = reserve_passes(c, 6u * (unsigned)std::min(o.max_sweeps, 1 << 20) + 12u);
     if (rc) return rc;
     const int tv = em ? kWaveTV : drift_tile_rows(g);
-    if ((rc = wave_scratch(c, g, tv))) return rc;
+    if ((rc = wave_scratch(c, g, tv, s))) return rc;
     cudaError_t e;
     if ((e = cudaMemsetAsync(c->w_counters, 0, 2 * sizeof(unsigned), s)) != cudaSuccess ||
         (e = cudaMemsetAsync(c->w_evaluated, 0, sizeof(unsigned long long), s)) != cudaSuccess)
@@ -638,7 +642,7 @@ static BatchCtlMem batch_ctl_mem(char *base, int n)
     return m;
 }
 
-static int batch_scratch(fold3d_ctx *c, const std::vector<fold3d_grid> &grids, int tv = kWaveTV)
+static int batch_scratch(fold3d_ctx *c, const std::vector<fold3d_grid> &grids, cudaStream_t s, int tv = kWaveTV)
 {
     const int n = (int)grids.size();
     std::vector<int> key(3 * (size_t)n);
@@ -692,7 +696,7 @@ static int batch_scratch(fold3d_ctx *c, const std::vector<fold3d_grid> &grids, i
     }
     cudaError_t e;
     if ((e = cudaMalloc(&c->b_scratch, words * 4)) != cudaSuccess ||
-        (e = cudaMemset(c->b_scratch, 0, words * 4)) != cudaSuccess ||
+        (e = cudaMemsetAsync(c->b_scratch, 0, words * 4, s)) != cudaSuccess ||
         (e = cudaMalloc(&c->b_slots, 2 * (size_t)n * 8)) != cudaSuccess)
         return set_errorf(FOLD3D_ERR_NOMEM, "batch scratch: %s", cudaGetErrorString(e));
     if (!c->b_counters && (e = cudaMalloc(&c->b_counters, 2 * sizeof(unsigned))) != cudaSuccess)
@@ -713,6 +717,7 @@ static int batch_scratch(fold3d_ctx *c, const std::vector<fold3d_grid> &grids, i
         cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, dev);
     }
     if (!c->batch_adj_bps) c->batch_adj_bps = batch_adj_blocks_per_sm(false);
+    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_error(e, "batch scratch");
     c->bkey = key;
     c->btv = tv;
     return FOLD3D_OK;
@@ -805,7 +810,7 @@ static int solve_batch_cfg(fold3d_ctx *c, int n, const SolveInst *in, bool f32, 
     if (rc) return rc;
     std::vector<fold3d_grid> grids(n);
     for (int i = 0; i < n; ++i) grids[i] = in[i].grid;
-    if ((rc = batch_scratch(c, grids, tv))) return rc;
+    if ((rc = batch_scratch(c, grids, s, tv))) return rc;
     cudaError_t e;
     const unsigned e0 = c->epoch + 1;
     const unsigned skip_from = o.skip ? e0 + 6 : 0xffffffffu;
@@ -1202,7 +1207,7 @@ static int adjoint_batch(fold3d_ctx *c, int n, const AdjInst *in, bool f32, int 
     if (rc) return rc;
     std::vector<fold3d_grid> grids(n);
     for (int i = 0; i < n; ++i) grids[i] = in[i].grid;
-    if ((rc = batch_scratch(c, grids))) return rc;
+    if ((rc = batch_scratch(c, grids, s))) return rc;
     std::vector<size_t> off(n + 1, 0);
     for (int i = 0; i < n; ++i) off[i + 1] = off[i] + field_cells(in[i].grid);
     if ((rc = adj_scratch(c, off[n]))) return rc;  // doubles: room for floats too
@@ -1621,7 +1626,7 @@ int fold3d_selftest_wait_timeout(fold3d_ctx *c, double timeout_ms)
     const fold3d_grid g = {16, 16, 16, 1.0, 1.0, 1.0};
     const fold3d_medium m = {1.1, -0.35, 0.4, 0.7};
     const int tv = drift_tile_rows(g);
-    int rc = wave_scratch(c, g, tv);
+    int rc = wave_scratch(c, g, tv, c->stream);
     if (rc) return rc;
     cudaError_t e;
     const size_t cells = field_cells(g);
