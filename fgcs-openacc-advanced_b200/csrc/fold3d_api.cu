@@ -167,10 +167,10 @@ struct fold3d_ctx {
     size_t d_field_cells = 0;
     // WAVEFRONT engine scratch, sized for the grid of key_wg
     fold3d_grid key_wg{};
-    int key_wtv = 0;                         // and tiles of this many rows
     unsigned *w_flags = nullptr;
-    int w_fshift = 0;                        // log2 of the words between two flags
+    int w_fshift = 0;                        // log2 of the words between two flags, last solve
     unsigned *w_mod[3] = {nullptr, nullptr, nullptr};
+    size_t w_flag_words = 0, w_mod_words[3] = {0, 0, 0};
     unsigned *w_counters = nullptr;          // [0] work, [1] status
     unsigned long long *w_evaluated = nullptr;
     unsigned epoch = 0;                      // passes run so far on this context (never decreases)
@@ -426,12 +426,31 @@ static int reserve_passes(fold3d_ctx *c, unsigned passes)
     return FOLD3D_OK;
 }
 
-// The clears run on the caller's stream, which need not wait for the legacy one,
-// and are over before the scratch counts as made.
+// The scratch of one grid serves every tile height: what an earlier layout left
+// in it are passes numbered below the ones to come, which neither release a wait
+// nor count as recent, so it is only made anew when it is too small (a drift
+// solve after an elliptical one, once).  The clears run on the caller's stream,
+// which need not wait for the legacy one, and are over before the scratch counts
+// as made.
 static int wave_scratch(fold3d_ctx *c, const fold3d_grid &g, int tv, cudaStream_t s)
 {
-    if (c->w_flags && c->key_wg.nx == g.nx && c->key_wg.ny == g.ny && c->key_wg.nz == g.nz && c->key_wtv == tv)
-        return FOLD3D_OK;
+    const int n[3] = {g.nx, g.ny, g.nz};
+    size_t flags = 0, mods[3];
+    for (int b = 0; b < 3; ++b) {
+        int ntu, ntv;
+        orient_tiles(g, b, ntu, ntv, tv);
+        flags = std::max(flags, (size_t)(n[b] - 1) * ntu * ntv);
+        mods[b] = (size_t)(n[b] + 2) * ntu * ntv;
+    }
+    c->w_fshift = (long long)flags <= kSpreadFlags ? 3 : 0;
+    flags <<= c->w_fshift;
+    if (c->w_flags && c->key_wg.nx == g.nx && c->key_wg.ny == g.ny && c->key_wg.nz == g.nz) {
+        if (flags <= c->w_flag_words && mods[0] <= c->w_mod_words[0] && mods[1] <= c->w_mod_words[1] &&
+            mods[2] <= c->w_mod_words[2])
+            return FOLD3D_OK;
+        flags = std::max(flags, c->w_flag_words);
+        for (int b = 0; b < 3; ++b) mods[b] = std::max(mods[b], c->w_mod_words[b]);
+    }
     if (c->w_flags) cudaFree(c->w_flags);
     for (int b = 0; b < 3; ++b) {
         if (c->w_mod[b]) cudaFree(c->w_mod[b]);
@@ -439,22 +458,13 @@ static int wave_scratch(fold3d_ctx *c, const fold3d_grid &g, int tv, cudaStream_
     }
     c->w_flags = nullptr;
     c->key_wg = fold3d_grid{};
-    const int n[3] = {g.nx, g.ny, g.nz};
-    size_t flag_words = 0;
     cudaError_t e;
-    for (int b = 0; b < 3; ++b) {
-        int ntu, ntv;
-        orient_tiles(g, b, ntu, ntv, tv);
-        flag_words = std::max(flag_words, (size_t)(n[b] - 1) * ntu * ntv);
-        const size_t words = (size_t)(n[b] + 2) * ntu * ntv;
-        if ((e = cudaMalloc(&c->w_mod[b], words * 4)) != cudaSuccess ||
-            (e = cudaMemsetAsync(c->w_mod[b], 0, words * 4, s)) != cudaSuccess)
+    for (int b = 0; b < 3; ++b)
+        if ((e = cudaMalloc(&c->w_mod[b], mods[b] * 4)) != cudaSuccess ||
+            (e = cudaMemsetAsync(c->w_mod[b], 0, mods[b] * 4, s)) != cudaSuccess)
             return set_errorf(FOLD3D_ERR_NOMEM, "wavefront scratch: %s", cudaGetErrorString(e));
-    }
-    c->w_fshift = (long long)flag_words <= kSpreadFlags ? 3 : 0;
-    flag_words <<= c->w_fshift;
-    if ((e = cudaMalloc(&c->w_flags, flag_words * 4)) != cudaSuccess ||
-        (e = cudaMemsetAsync(c->w_flags, 0, flag_words * 4, s)) != cudaSuccess)
+    if ((e = cudaMalloc(&c->w_flags, flags * 4)) != cudaSuccess ||
+        (e = cudaMemsetAsync(c->w_flags, 0, flags * 4, s)) != cudaSuccess)
         return set_errorf(FOLD3D_ERR_NOMEM, "wavefront scratch: %s", cudaGetErrorString(e));
     if (!c->w_counters) {
         if ((e = cudaMalloc(&c->w_counters, 2 * sizeof(unsigned))) != cudaSuccess ||
@@ -467,7 +477,8 @@ static int wave_scratch(fold3d_ctx *c, const fold3d_grid &g, int tv, cudaStream_
         cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, dev);
     }
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_error(e, "wavefront scratch");
-    c->key_wtv = tv;
+    c->w_flag_words = flags;
+    for (int b = 0; b < 3; ++b) c->w_mod_words[b] = mods[b];
     c->key_wg = g;  // fresh flags and maps are zero, below every pass number to come
     return FOLD3D_OK;
 }
