@@ -1038,7 +1038,7 @@ static int batch_config(fold3d_ctx *c, int n, const SolveInst *in, bool f32, cud
         return FOLD3D_OK;
     }
     if (n < 8) {  // too few instances to be worth a tuning run
-        tv = kWaveTV;
+        tv = std::max(kWaveTV, 2);  // batched passes have 2, 4 or 8 rows
         bps = batch_occupancy_of(c, f32, tv);
         return FOLD3D_OK;
     }

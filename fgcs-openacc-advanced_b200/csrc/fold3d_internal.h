@@ -122,8 +122,8 @@ static_assert(kBatchChunk >= 1 && kBatchChunk <= 32, "batch chunk");
 #endif
 
 // WAVEFRONT tiles are 32 points along the plane's faster axis by some rows:
-// FOLD3D_WAVE_TV in single solves of the elliptical medium, where one CTA of
-// 32*FOLD3D_WAVE_TV threads works on a tile.
+// FOLD3D_WAVE_TV (1, 2, 4 or 8) in single solves of the elliptical medium, where
+// one CTA of 32*FOLD3D_WAVE_TV threads works on a tile.
 #ifndef FOLD3D_WAVE_TV
 #define FOLD3D_WAVE_TV 4
 #endif

@@ -57,12 +57,12 @@ __device__ __forceinline__ bool bits_differ(float a, float b) { return __float_a
 
 }  // namespace
 
-constexpr int kWaveThreads = 128;  // four warps
-
+constexpr int kWaveThreads = 128;           // the drift medium's CTAs: four warps
+constexpr int kEllipThreads = 32 * kWaveTV;  // the elliptical medium's: a warp per row of the tile
 
 template <class R> constexpr int wave_min_blocks()
 {
-    return sizeof(R) == 8 ? FOLD3D_WAVE_MINB_ELLIP : FOLD3D_WAVE_MINB_ELLIP_F32;
+    return (sizeof(R) == 8 ? FOLD3D_WAVE_MINB_ELLIP : FOLD3D_WAVE_MINB_ELLIP_F32) * 4 / kWaveTV;
 }
 
 // A lane's point (u, v) of the target plane src + sg: update it from the source
@@ -389,11 +389,11 @@ __global__ void __launch_bounds__(kWaveThreads, FOLD3D_WAVE_MINB_DRIFT)
 // both is the chain from step to step, and on x-normal planes loads of which
 // every lane's is a sector of its own (2 to 3 times a k pass at 512^3).
 template <class R>
-__global__ void __launch_bounds__(kWaveThreads, wave_min_blocks<R>())
+__global__ void __launch_bounds__(kEllipThreads, wave_min_blocks<R>())
     wave_item_kernel(R *__restrict__ T, WaveArgs a, const __grid_constant__ EllipParam tab)
 {
     __shared__ int s_next;
-    __shared__ double s_fan[sizeof(R) == 8 ? 9 * kWaveThreads : 1];
+    __shared__ double s_fan[sizeof(R) == 8 ? 9 * kEllipThreads : 1];
     const long long total = (long long)a.steps * a.ntu * a.ntv;
     double dmax = 0.0;
     unsigned evaluated = 0;
@@ -415,14 +415,13 @@ __global__ void __launch_bounds__(kWaveThreads, wave_min_blocks<R>())
     wave_flush<kWaveTV>(dmax, evaluated, a.maxd, a.evaluated);
 }
 
-__global__ void __launch_bounds__(kWaveThreads, wave_min_blocks<double>())
+__global__ void __launch_bounds__(kEllipThreads, wave_min_blocks<double>())
     wave_pass_kernel(double *__restrict__ T, WaveArgs a, const __grid_constant__ EllipParam tab)
 {
-    constexpr int TV = kWaveTV, kWarps = kWaveThreads / 32;
-    static_assert(kWarps == TV && TV >= 3, "one row per warp");
+    constexpr int TV = kWaveTV, kWarps = TV, kPublisher = TV > 1 ? 32 : 0;  // a warp other than 0, where there is one
     __shared__ int s_item[2];           // the CTA's items, by parity; -1 for none
     __shared__ int s_state;             // 0 update, 1 skip, 2 a wait gave up
-    __shared__ double s_fan[9 * kWaveThreads];
+    __shared__ double s_fan[9 * kEllipThreads];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ntiles = a.ntu * a.ntv;
     const unsigned total = (unsigned)(a.steps * ntiles);
@@ -470,15 +469,15 @@ __global__ void __launch_bounds__(kWaveThreads, wave_min_blocks<double>())
         if (state == 2) break;
         bool changed = false;
         if (state == 0)
-            changed = ellip_point<double>(T, a, tab, src, u, tv * TV + warp + 1, s_fan + threadIdx.x, kWaveThreads, dmax,
-                                     evaluated);
+            changed = ellip_point<double>(T, a, tab, src, u, tv * TV + warp + 1, s_fan + threadIdx.x, kEllipThreads,
+                                          dmax, evaluated);
         if (changed) {
             wave_mark<1, TV>(a, u, tv * TV + warp + 1, tgt);
             wave_mark<2, TV>(a, u, tv * TV + warp + 1, tgt);
         }
         if (claims) s_item[slot ^ 1] = (claim < total) ? (int)claim : -1;
         const bool any = __syncthreads_or(changed);  // precedes the release: every thread's stores come before the flag
-        if (threadIdx.x == 32) {
+        if (threadIdx.x == kPublisher) {
             st_release(a.flags + ((long long)item << a.fshift), want | (any ? 1u : 0u));
             if (any) a.mod[0][(long long)tgt * ntiles + t] = a.epoch;
         }
@@ -674,29 +673,31 @@ cudaError_t launch_wave_pass(double *T, const WaveArgs &a, const DirTable &tab, 
 cudaError_t launch_wave_pass_ellip(void *T, bool f32, const WaveArgs &a, const EllipParam &p, int grid, cudaStream_t s,
                                    bool large)
 {
-    if (f32) wave_item_kernel<float><<<grid, kWaveThreads, 0, s>>>(static_cast<float *>(T), a, p);
-    else if (large) wave_pass_kernel<<<grid, kWaveThreads, 0, s>>>(static_cast<double *>(T), a, p);
-    else wave_item_kernel<double><<<grid, kWaveThreads, 0, s>>>(static_cast<double *>(T), a, p);
+    if (f32) wave_item_kernel<float><<<grid, kEllipThreads, 0, s>>>(static_cast<float *>(T), a, p);
+    else if (large) wave_pass_kernel<<<grid, kEllipThreads, 0, s>>>(static_cast<double *>(T), a, p);
+    else wave_item_kernel<double><<<grid, kEllipThreads, 0, s>>>(static_cast<double *>(T), a, p);
     return cudaGetLastError();
 }
 
-template <class K> static int occupancy(K kernel)
+template <class K> static int occupancy(K kernel, int threads)
 {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kWaveThreads, 0) != cudaSuccess) return 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, 0) != cudaSuccess) return 1;
     return n > 0 ? n : 1;
 }
 
 int wave_blocks_per_sm(bool f32, bool large)
 {
-    return f32 ? occupancy(wave_item_kernel<float>) : large ? occupancy(wave_pass_kernel)
-                                                            : occupancy(wave_item_kernel<double>);
+    return f32     ? occupancy(wave_item_kernel<float>, kEllipThreads)
+           : large ? occupancy(wave_pass_kernel, kEllipThreads)
+                   : occupancy(wave_item_kernel<double>, kEllipThreads);
 }
 
 int drift_blocks_per_sm(int tv)
 {
-    return tv == 1 ? occupancy(drift_pass_kernel<1>) : tv == 2 ? occupancy(drift_pass_kernel<2>)
-                                                               : occupancy(drift_pass_kernel<4>);
+    return tv == 1   ? occupancy(drift_pass_kernel<1>, kWaveThreads)
+           : tv == 2 ? occupancy(drift_pass_kernel<2>, kWaveThreads)
+                     : occupancy(drift_pass_kernel<4>, kWaveThreads);
 }
 
 }  // namespace fold3d
