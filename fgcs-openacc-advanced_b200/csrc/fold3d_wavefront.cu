@@ -496,10 +496,13 @@ __global__ void __launch_bounds__(kEllipThreads, wave_min_blocks<double>())
 // spread over many instances at once.
 // ---------------------------------------------------------------------------
 // Resident CTAs per SM the batched kernel is compiled for, by tile height: the
-// same register budget per thread for every height.
+// option's warps, rounded up to whole CTAs.  FP64 at 8 rows gets 3 CTAs and 80
+// registers per thread, at 2 and 4 rows 20 warps and 96; rounded down it had 16
+// warps (ms at 8 rows, 2 and 3 CTAs: 24 instances of 96 to 200 points per axis
+// 328, 299; 48 of 64 to 176 395, 341; at 4 rows 280 and 323).
 template <class R, int TV> constexpr int batch_min_blocks()
 {
-    return (sizeof(R) == 8 ? FOLD3D_WAVE_MINB_BATCH : FOLD3D_WAVE_MINB_BATCH_F32) * 4 / TV;
+    return ((sizeof(R) == 8 ? FOLD3D_WAVE_MINB_BATCH : FOLD3D_WAVE_MINB_BATCH_F32) * 4 + TV - 1) / TV;
 }
 
 template <class R, int TV>
