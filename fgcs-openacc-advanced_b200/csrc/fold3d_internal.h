@@ -99,11 +99,14 @@ enum Variant {
 constexpr unsigned kPollNs = FOLD3D_POLL_NS;
 
 // Passes of at most this many items have a 32-byte sector for each completion
-// flag (128 MB at most): the many waiting warps and CTAs poll a step's few
-// flags, and 32 of them in one line are served one after another.  ms, 4 and 32
-// bytes per flag: drift 256^3, 8 sweeps from the host 128, 116; float32 TTI
-// 380x319x257 69.7, 63.9; 512^3 346, 347 (more flags than this).
-constexpr long long kSpreadFlags = 1ll << 22;
+// flag (64 MB at most): the many waiting warps and CTAs poll a step's few flags,
+// and 32 of them in one line are served one after another.  Larger passes have
+// more work between two polls of a line and gain nothing.  ms, 4 and 32 bytes per
+// flag, drift, 4 sweeps: 256^3 (0.5 M items) 63.9, 57.4; 320^3 (1.0 M) 86.3, 78.5;
+// 400^3 (2.1 M) 115.4, 113.1; 448^3 (2.8 M) 141.1, 140.3; 512^3 (4.2 M) 191.3,
+// 192.6; float32 TTI 380x319x257 69.7, 63.9; 36 FP64 TTI instances of 184 to 200
+// points per axis (2 M) 787, 793.
+constexpr long long kSpreadFlags = 1ll << 21;
 
 // Items a batched pass's CTA claims at a time: two, or four when a plane step of
 // the batch has kBatchBusy tiles or more for every resident CTA.  Few, and every
