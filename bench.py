@@ -264,6 +264,7 @@ def run_reference(args):
         threads = host_threads()
         os.environ["OMP_NUM_THREADS"] = str(threads)
         r = RefLib(n, omp=True)
+        r.L  # loads it, or says here why it cannot
         if n <= 640:
             T0 = r.init_implicit()  # the reference's own ImplicitInitialiser
             setup = "starting field from the reference's own ImplicitInitialiser"

@@ -260,24 +260,12 @@ _REF_CALLS = (
 
 
 class RefLib:
-    """The reference's own code built for the host at size n (oracle/_ref)."""
+    """The reference's own code built for the host at size n (oracle/_ref),
+    built and loaded when it is first called; the reference driver's argument
+    lists need neither."""
 
     def __init__(self, n: int, omp: bool = False):
-        from . import build
-
-        path = build.ref_lib_path(n, omp)
-        if not os.path.exists(path):
-            build.build_ref(n)
-        self.n = n
-        L = C.CDLL(path)
-        L.ImplicitInitialiser.argtypes = [_ptr, _int, _int, _int, _dbl, _dbl, _dbl]
-        L.InitFoldFromPoint.argtypes = [_dbl] * 7
-        L.InitFoldFromPoint.restype = _dbl
-        L.ImpSurfF.argtypes = [_dbl] * 3
-        L.ImpSurfF.restype = _dbl
-        for name, *_ in _REF_CALLS:
-            getattr(L, name).argtypes = [_ptr, _int] + [_dbl] * 10
-        self.L = L
+        self.n, self.omp, self._L = n, omp, None
         DX = dy = dz = ref_spacing(n)
         self.sp = {
             "DX": DX, "dy": dy, "dz": dz,
@@ -286,6 +274,25 @@ class RefLib:
             "DYZP": math.sqrt(dy * dy + dz * dz),
         }
         self.const = {"x": REF_A[0], "y": REF_A[1], "z": REF_A[2]}
+
+    @property
+    def L(self):
+        if self._L is None:
+            from . import build
+
+            path = build.ref_lib_path(self.n, self.omp)
+            if not os.path.exists(path):
+                build.build_ref(self.n)
+            L = C.CDLL(path)
+            L.ImplicitInitialiser.argtypes = [_ptr, _int, _int, _int, _dbl, _dbl, _dbl]
+            L.InitFoldFromPoint.argtypes = [_dbl] * 7
+            L.InitFoldFromPoint.restype = _dbl
+            L.ImpSurfF.argtypes = [_dbl] * 3
+            L.ImpSurfF.restype = _dbl
+            for name, *_ in _REF_CALLS:
+                getattr(L, name).argtypes = [_ptr, _int] + [_dbl] * 10
+            self._L = L
+        return self._L
 
     def init_implicit(self) -> np.ndarray:
         n = self.n

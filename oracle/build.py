@@ -75,6 +75,10 @@ def build_oracle(force: bool = False) -> str:
     return out
 
 
+class ReferenceMissing(RuntimeError):
+    """The reference's sources are not here to build."""
+
+
 def reference_available() -> bool:
     return os.path.isfile(os.path.join(REF_DIR, "AN_ISO_1_OpenACC.c"))
 
@@ -119,7 +123,7 @@ def _omp_transform(outdir: str) -> str:
 def build_ref(n: int, with_program: bool = False, force: bool = False) -> str:
     """Build oracle/_ref/n<n>/{libref.so, libref_omp.so[, an_iso_1_ref]}."""
     if not reference_available():
-        raise RuntimeError("reference sources not found under %s" % REF_ROOT)
+        raise ReferenceMissing("reference sources not found under %s" % REF_ROOT)
     outdir = os.path.join(REF_OUT, "n%d" % n)
     os.makedirs(outdir, exist_ok=True)
     acc = os.path.join(REF_DIR, "AN_ISO_1_OpenACC.c")
@@ -161,7 +165,7 @@ def build_dropin(n: int = 128, force: bool = False) -> str:
     ImplicitInitialiser and the acc_* runtime calls resolve to the library
     (the reference's Fold3dPMM.c is not linked).  Needs libfold3dpmm.so."""
     if not reference_available():
-        raise RuntimeError("reference sources not found under %s" % REF_ROOT)
+        raise ReferenceMissing("reference sources not found under %s" % REF_ROOT)
     root = os.path.dirname(HERE)
     pkg = os.path.join(root, "fgcs-openacc-advanced_b200")
     lib = os.path.join(pkg, "libfold3dpmm.so")
