@@ -245,6 +245,17 @@ def single_thread_reference(T0, n, seconds=3.0):
         return {"single_thread_value": None, "single_thread_sample": "unavailable: %s" % str(e).splitlines()[0]}
 
 
+def fp64_capture(n):
+    """The FP64 pipe's and the issue slots' share of the active cycles
+    (profiles/drift_pass_kernel_1280_planes.md): a capture of the form with
+    tiles of 4 rows, which cubic grids of 32000 rows of 32 points a plane step
+    or more run (drift_tile_rows in fold3d_api.cu); None for the others."""
+    if n * n / 32.0 < 32000.0:
+        return None
+    return {"pct_of_active_cycles": 9.5, "issue_active_pct": 59.0, "kernel": "drift_pass_kernel<4>",
+            "capture": "k_up and x_down passes over 1280^2 planes (mean), settled field"}
+
+
 def run_reference(args):
     """--impl reference: rank 0 only."""
     import numpy as np
@@ -1101,13 +1112,11 @@ def main():
     # DRAM bytes per launch: the bytes per update that ncu measured
     # (profiles/wave_pass_kernel_fold512_full.md; an older kernel, which read
     # and wrote the same values) times this launch's updates, and the FP64
-    # pipe's share of the active cycles from a capture of this kernel over
-    # 1280^2 planes (profiles/drift_pass_kernel_1280_planes.md)
+    # pipe's share of the active cycles where this kernel's form was captured
     wave = rep.engine == f3d.ENGINE_WAVEFRONT
     upd_launch = upd / launches_per_step
     traffic = WAVE_DRAM_BYTES_PER_UPDATE * upd_launch if wave else None
-    fp64 = {"pct_of_active_cycles": 9.5, "issue_active_pct": 59.0,
-            "capture": "k_up and x_down passes over 1280^2 planes (mean), settled field"} if wave else None
+    fp64 = fp64_capture(n) if wave else None
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": traffic, "peak_kind": peak_kind,
                 "kernel": "plane_kernel" if rep.engine == f3d.ENGINE_PLANES else "drift_pass_kernel",
