@@ -363,7 +363,8 @@ __host__ __device__ __forceinline__ R point_update_ellip(R told, R st, const R n
 // their own size, so candidates that the filter tells apart often tie.
 //
 // ms before (gated FP64 candidates) and now, with the passes' other changes of
-// the time (waits, barriers, batch chunks): TTI 512^3 to 1e-10 374, 248; 24
+// the time (waits, barriers, batch chunks), one source each (a 512^3 solve takes
+// 190 to 310 by where its source lies): TTI 512^3 to 1e-10 374, 248; 24
 // instances of 96 to 200 points per axis 476, 264; 8 sources at 192^3 with their gradients 471,
 // 249; 128^3 14.3, 12.5.  A point now costs 0.3 to 0.4 FP64 candidates of the
 // 33; what bounds a pass is in fold3d_wavefront.cu.

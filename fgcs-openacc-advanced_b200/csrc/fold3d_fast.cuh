@@ -76,8 +76,9 @@
 //    to 150 FP64 instructions of which most depend on one another, and in a
 //    settled field it nearly always ends in a rejection: over 192^3 sweeps of
 //    the reference's workload a warp row enters 4.5 bodies and 0.17 of its
-//    points improve; with the filter it enters 0.4.  So every gate and every body is first judged in float,
-//    from differences rounded once: c_r = float(st - s_r), E = float(tn - st).
+//    points improve; with the filter it enters 0.4.  So every gate and every
+//    body is first judged in float, from differences rounded once:
+//    c_r = float(st - s_r), E = float(tn - st).
 //
 //    Gates.  tn - min(sources) = E + max(c), so a call can only matter when
 //    E + max(c) > B (its skip bound; an edge's fall-back when E + c > K,

@@ -134,13 +134,15 @@ constexpr int kWaveTV = FOLD3D_WAVE_TV;
 
 // Resident 128-thread CTAs per SM the forward dataflow kernels are compiled for
 // (their register budget is 65536 / (128 * this)); build options, each the
-// count that measured fastest.  Drift: 4 (128 registers; ms at 512^3, 8 sweeps,
-// and 1280^3, 2 sweeps, for 3, 4, 5 and 6: 342, 342, 333, 352 and 1269, 1126,
-// 1158, 1168): the update is one long chain per point, which spills and
-// reloads below 100 registers lengthen.  The FP64 elliptical medium 5 (128^3
-// and 512^3 to 1e-10, for 4, 5 and 6: 12.7, 12.7, 13.0 and 317, 312, 328); the
-// float32 one 8; FP64 batches 5 (24 instances of 96 to 200 points per axis, for
-// 4, 5, 6 and 8: 327, 327, 340, 377), float32 batches 8.
+// count that measured fastest.  Drift: 4 for its three tile heights (128
+// registers; ms for 3, 4, 5 and 6: 1280^3, 2 sweeps, tiles of 4 rows 1269, 1126,
+// 1158, 1168; 512^3, 8 sweeps, tiles of 1 row 342, 342, 333, 352, where 5 would be
+// 3% faster): the update is one long chain per point, which spills and reloads
+// below 100 registers lengthen.  The FP64 elliptical medium 5 (128^3 and 512^3 to
+// 1e-10, for 4, 5 and 6: 12.7, 12.7, 13.0 and 317, 312, 328); the float32 one 8;
+// FP64 batches 5 (for 5, 6 and 8, claims in chunks of two: 24 instances of 96 to
+// 200 points per axis 277, 275, 309; 48 of 96 to 256 784, 773, 804; 64 of 176^3 918,
+// 875, 852: mixed), float32 batches 8.
 #ifndef FOLD3D_WAVE_MINB_DRIFT
 #define FOLD3D_WAVE_MINB_DRIFT 4
 #endif

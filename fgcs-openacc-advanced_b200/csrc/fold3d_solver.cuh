@@ -10,11 +10,14 @@
 //
 // Structure of the update (used by the skipping and reordering logic in the
 // kernels): every candidate a solver can accept is strictly greater than the
-// minimum of the previous-plane values it is built from, and every early
-// return only fires when no candidate could beat the current time.  The
-// result of a point update is therefore min(T_old, M(neighbours)), where
-// M depends on the nine previous-plane values and on the side (sign) of the
-// target only.
+// minimum of the previous-plane values it is built from, and the solvers' own
+// early returns only fire when no candidate could beat the current time.  The
+// update's early exit (:231) is not of that kind: it compares the time after the
+// 1-D candidate with seven of the nine values and leaves all the solvers out.
+// Behind it, a point update is min(T_old, M(neighbours)), where M depends on the
+// nine previous-plane values and on the side (sign) of the target only; and a
+// point whose neighbours are as they were keeps its value either way, since a
+// lower time takes the exit wherever a higher one did.
 #pragma once
 #include <cstdint>
 

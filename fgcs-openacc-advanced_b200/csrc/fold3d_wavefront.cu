@@ -384,8 +384,8 @@ __global__ void __launch_bounds__(kWaveThreads, FOLD3D_WAVE_MINB_DRIFT)
 // rows run between them; after the second, warp 1 publishes the item while the
 // others go on.  On smaller planes, and for float fields, the plane-to-plane
 // chain binds and wave_item_kernel is faster, where thread 0 publishes before
-// anything of the next item begins (ms; two barriers, this: 128^3 to 1e-10
-// 12.7, 12.2; 512^3 312, 339; float32 380x319x257 72.4, 69.8).  What bounds
+// anything of the next item begins (ms; two barriers, this, one source each:
+// 128^3 to 1e-10 12.7, 12.2; 512^3 312, 339; float32 380x319x257 72.4, 69.8).  What bounds
 // both is the chain from step to step, and on x-normal planes loads of which
 // every lane's is a sector of its own (2 to 3 times a k pass at 512^3).
 template <class R>
