@@ -118,11 +118,12 @@ constexpr int kBatchChunk = 4;
 constexpr int kBatchBusy = 10;
 static_assert(kBatchChunk >= 1 && kBatchChunk <= 32, "batch chunk");
 
-// Rows of the drift medium's tiles; build option, 0: by grid size
-// (drift_tile_rows in fold3d_api.cu).
+// Rows of the drift medium's tiles; build option: 1, 2 or 4, the heights its
+// passes are compiled for, or 0: by grid size (drift_tile_rows in fold3d_api.cu).
 #ifndef FOLD3D_DRIFT_TV
 #define FOLD3D_DRIFT_TV 0
 #endif
+static_assert(FOLD3D_DRIFT_TV == 0 || FOLD3D_DRIFT_TV == 1 || FOLD3D_DRIFT_TV == 2 || FOLD3D_DRIFT_TV == 4, "drift tile rows");
 
 // WAVEFRONT tiles are 32 points along the plane's faster axis by some rows:
 // FOLD3D_WAVE_TV (1, 2, 4 or 8) in single solves of the elliptical medium, where
